@@ -574,6 +574,7 @@ nw_status nw_ctx_destroy(nw_ctx* ctx) {
     if (b) cudaFree(b);
   if (ctx->d_fockp) cudaFree(ctx->d_fockp);
   free_buf(ctx->build_work);
+  free_buf(ctx->build_tasks);
   free_buf(ctx->bt_dets);
   free_buf(ctx->bt_desc);
   free_buf(ctx->bt_pairs);

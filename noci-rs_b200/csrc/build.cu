@@ -436,6 +436,147 @@ inline int grid_for(size_t work, int block = 256) {
   return (int)g;
 }
 
+// Slab offsets of a fast pair's pieces.
+struct FastOff {
+  size_t recx[2], recy[2], jas[2], ii0;
+};
+
+// Four-index tensors of a build on the fused route: first halves (A, B), each with the second halves
+// that read it.  Tensors that subtract from a J slot run after all that store.
+struct FusedPlan {
+  struct Second {
+    const double* c;
+    const double* d;
+    double* out;
+  };
+  struct Half {
+    const double* a;
+    const double* b;
+    std::vector<Second> full;
+  };
+  std::vector<Half> phase[2];  // kStore, kSubtract
+  void add(bool subtract, const double* a, const double* b, const double* c, const double* d, double* out) {
+    std::vector<Half>& v = phase[subtract ? 1 : 0];
+    size_t i = 0;
+    while (i < v.size() && !(v[i].a == a && v[i].b == b)) ++i;
+    if (i == v.size()) v.push_back(Half{a, b, {}});
+    v[i].full.push_back(Second{c, d, out});
+  }
+};
+
+// Runs the halves of one phase in batches whose first halves fit `cap` doubles at `work`.
+nw_status run_halves(nw_ctx* ctx, const std::vector<FusedPlan::Half>& halves, int mode, int n, double* work, size_t cap) {
+  const size_t hsz = (size_t)n * n * packed_ld(n), per = std::max<size_t>(1, cap / hsz);
+  std::vector<TransformTask> tasks;
+  struct Batch {
+    size_t h0, nh, f0, nf;
+  };
+  std::vector<Batch> batches;
+  for (size_t i = 0; i < halves.size(); i += per) {
+    Batch b{tasks.size(), std::min(per, halves.size() - i), 0, 0};
+    for (size_t k = 0; k < b.nh; ++k)
+      tasks.push_back(TransformTask{ctx->d_eri, halves[i + k].a, halves[i + k].b, work + k * hsz, 0, 0});
+    b.f0 = tasks.size();
+    for (size_t k = 0; k < b.nh; ++k)
+      for (const auto& f : halves[i + k].full)
+        tasks.push_back(TransformTask{work + k * hsz, f.c, f.d, f.out, mode, 0});
+    b.nf = tasks.size() - b.f0;
+    batches.push_back(b);
+  }
+  if (tasks.empty()) return NW_OK;
+  // the previous phase's kernels read the same table: the pageable copy below is ordered behind them
+  nw_status st = ensure(ctx, ctx->build_tasks, tasks.size() * sizeof(TransformTask));
+  if (st != NW_OK) return st;
+  TransformTask* d = static_cast<TransformTask*>(ctx->build_tasks.p);
+  NW_CUDA(ctx, cudaMemcpyAsync(d, tasks.data(), tasks.size() * sizeof(TransformTask), cudaMemcpyHostToDevice, 0));
+  for (const Batch& b : batches) {
+    NW_DG(ctx, two_sided(0, true, d + b.h0, (int)b.nh, n));
+    NW_DG(ctx, two_sided(0, false, d + b.f0, (int)b.nf, n));
+  }
+  return NW_OK;
+}
+
+template <typename T>
+nw_status upload_tasks(nw_ctx* ctx, const std::vector<T>& v, T** out) {
+  nw_status st = ensure(ctx, ctx->build_tasks, v.size() * sizeof(T));
+  if (st != NW_OK) return st;
+  *out = static_cast<T*>(ctx->build_tasks.p);
+  NW_CUDA(ctx, cudaMemcpyAsync(*out, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, 0));
+  return NW_OK;
+}
+
+// The fused route: J and II of every resident pair.  Without zero-overlap orbitals the intermediates
+// of (w, x) are those of (x, w) with rows and columns exchanged (M -> M^T), so only x <= w is
+// transformed and the other is a permuted copy; and the exchange part of the antisymmetrised J cancels
+// (it is symmetric in the columns that are exchanged), leaving N[ab|cd] - N[ad|cb].  `plan` holds
+// the tensors of the pairs with zero-overlap orbitals.
+template <typename Res, typename F1, typename F2>
+nw_status run_fused(nw_ctx* ctx, FusedPlan& plan, int n, int nref, const Res& resident, const std::vector<char>& generic,
+                    const std::vector<FastOff>& fo, const F1& CX, const F2& XC, double* S0, double* work, size_t cap) {
+  const size_t n4 = (size_t)n * n * n * n, n4r = (n4 + 31) / 32 * 32;
+  const int o[2] = {ctx->nocc_a, ctx->nocc_b};
+  std::vector<double*> anti;
+  std::vector<MirrorTask> mirror;
+  std::vector<int> orphans;  // w > x resident without its mirror image (a block of a blocked evaluation)
+  auto tensors = [&](int p, double* const* dst, FusedPlan& pl) {
+    for (int s = 0; s < 2; ++s)
+      if (dst[s]) pl.add(false, CX(2 * p + s, 0), XC(2 * p + s, 0), CX(2 * p + s, 0), XC(2 * p + s, 0), dst[s]);
+    if (dst[2]) pl.add(false, CX(2 * p, 0), XC(2 * p, 0), CX(2 * p + 1, 0), XC(2 * p + 1, 0), dst[2]);
+  };
+  for (int x = 0; x < nref; ++x)
+    for (int w = 0; w < nref; ++w) {
+      const int p = x * nref + w, q = w * nref + x;
+      if (!resident(p) || generic[p]) continue;
+      if (x > w) {
+        if (!resident(q)) {
+          orphans.push_back(p);
+          continue;
+        }
+        for (int s = 0; s < 2; ++s) mirror.push_back(MirrorTask{S0 + fo[q].jas[s], S0 + fo[p].jas[s], o[s], o[s]});
+        mirror.push_back(MirrorTask{S0 + fo[q].ii0, S0 + fo[p].ii0, o[0], o[1]});
+        continue;
+      }
+      double* dst[3] = {S0 + fo[p].jas[0], S0 + fo[p].jas[1], S0 + fo[p].ii0};
+      tensors(p, dst, plan);
+      anti.push_back(dst[0]);
+      anti.push_back(dst[1]);
+    }
+  nw_status st = run_halves(ctx, plan.phase[0], kStore, n, work, cap);
+  if (st == NW_OK) st = run_halves(ctx, plan.phase[1], kSubtract, n, work, cap);
+  if (st != NW_OK) return st;
+  if (!anti.empty()) {
+    double** d = nullptr;
+    if ((st = upload_tasks(ctx, anti, &d)) != NW_OK) return st;
+    NW_CUDA(ctx, antisymmetrise(0, d, (int)anti.size(), n));
+  }
+  if (!mirror.empty()) {
+    MirrorTask* d = nullptr;
+    if ((st = upload_tasks(ctx, mirror, &d)) != NW_OK) return st;
+    NW_CUDA(ctx, mirror_tensors(0, d, (int)mirror.size(), n));
+  }
+  for (int p : orphans) {
+    const int x = p / nref, w = p % nref, q = w * nref + x;
+    for (int k = 0; k < 3; ++k) {  // one tensor at a time through one n^4 scratch
+      double* dst[3] = {nullptr, nullptr, nullptr};
+      dst[k] = work;
+      FusedPlan one;
+      tensors(q, dst, one);
+      if ((st = run_halves(ctx, one.phase[0], kStore, n, work + n4r, cap - n4r)) != NW_OK) return st;
+      if (k < 2) {
+        double** d = nullptr;
+        if ((st = upload_tasks(ctx, std::vector<double*>{work}, &d)) != NW_OK) return st;
+        NW_CUDA(ctx, antisymmetrise(0, d, 1, n));
+      }
+      MirrorTask* d = nullptr;
+      const std::vector<MirrorTask> m{MirrorTask{work, S0 + (k < 2 ? fo[p].jas[k] : fo[p].ii0), o[k < 2 ? k : 0],
+                                                 o[k < 2 ? k : 1]}};
+      if ((st = upload_tasks(ctx, m, &d)) != NW_OK) return st;
+      NW_CUDA(ctx, mirror_tensors(0, d, 1, n));
+    }
+  }
+  return NW_OK;
+}
+
 }  // namespace
 
 cudaError_t swap_qr(cudaStream_t st, const double* src, int n, double* dst) {
@@ -464,8 +605,13 @@ nw_status build_all(nw_ctx* ctx, const std::vector<char>* subset) {
                         4 * n2 /*X Y*/ + 2 * n2 /*tmp*/ + 2 * n2 /*JK*/ + 2 * n2 /*Jc*/ + 4 * n2 /*Fh*/ +
                         8 * n2 /*V*/ + 8 * n2 /*vab or vba*/ + 2 * n2 /*hxc*/ + 4 * n2 /*JKxc*/ +
                         4 * n2 /*JcXc*/ + 64;
+  const int nhalf_max = 16 * npair;  // first halves of the fused transforms, all pairs
+  const size_t half = n2 * packed_ld(n);
+  // the fused transforms hold at least eight first halves (half a tensor each) and one whole tensor; a
+  // small system holds them all, so that each stage is one launch
+  const size_t tensor_work = std::max<size_t>(8 * half + n4, std::min<size_t>(nhalf_max * half + n4, 8u << 20));
   // 40 arena pieces, each rounded up to 256 bytes
-  const size_t work_doubles = per_ps * nps + 5 * n4 + 40 * 32 + 4096;
+  const size_t work_doubles = per_ps * nps + n4 + std::max<size_t>(4 * n4 + 128, tensor_work) + 40 * 32 + 4096;
   // the workspace stays with the context, so rebuilds (blocked evaluation, transform changes)
   // do not allocate it again
   Arena ar;
@@ -505,11 +651,22 @@ nw_status build_all(nw_ctx* ctx, const std::vector<char>* subset) {
   double* JKxc = ar.take((size_t)nps * 4 * n2);
   double* JcXc = ar.take((size_t)nps * 4 * n2);
   double* G = ar.take(n4);
-  double* tA = ar.take(n4);
-  double* tB = ar.take(n4);
-  double* tD = ar.take(n4);
-  double* tE = ar.take(n4);
-  if (!tE) return fail(ctx, NW_ERR_ALLOC, "build workspace too small");
+  // four-index scratch: three tensors of the quarter-transform route, or the first halves of the fused one
+  const size_t tensors = std::max<size_t>(4 * n4 + 128, tensor_work);
+  double* tA = ar.take(tensors);
+  if (!tA) return fail(ctx, NW_ERR_ALLOC, "build workspace too small");
+  const size_t n4r = (n4 + 31) / 32 * 32;
+  double* tD = tA + n4r;
+  double* tE = tD + n4r;
+  // Route of the four-index tensors.  The fused half transforms need the tensor's permutation symmetry
+  // (checked once per context, to rounding: 32 ulp of the largest element) and n <= kTwoSidedMax, the
+  // matrices that fit shared memory; otherwise the quarter transforms (or a Cholesky route) run.
+  if (ctx->transform == NW_TRANSFORM_FP64 && ctx->eri_symmetric < 0) {
+    double big = 0.0, off = 0.0;
+    NW_CUDA(ctx, eri_symmetry(h, ctx->d_eri, n, G, &big, &off));
+    ctx->eri_symmetric = off <= 32 * 2.220446049250313e-16 * big ? 1 : 0;
+  }
+  const bool fused = ctx->transform == NW_TRANSFORM_FP64 && n <= kTwoSidedMax && ctx->eri_symmetric == 1;
   // Cholesky route of the four-index tensors (nw_set_transform)
   CholWork cw{};
   CholWork* cwp = nullptr;
@@ -675,9 +832,6 @@ nw_status build_all(nw_ctx* ctx, const std::vector<char>* subset) {
   struct GenOff {
     size_t x[2][2], y[2][2], fh[2][4], v[2][8], j[2][10], vab[8], vba[8], ii[16];
   };
-  struct FastOff {
-    size_t recx[2], recy[2], jas[2], ii0;
-  };
   std::vector<FastOff> fo(npair);
   std::vector<GenOff> go(npair);
   for (int p = 0; p < npair; ++p) {
@@ -742,11 +896,12 @@ nw_status build_all(nw_ctx* ctx, const std::vector<char>* subset) {
   std::vector<GenPair> hgen(npair);
   std::memset(hfast.data(), 0, sizeof(FastPair) * npair);
   std::memset(hgen.data(), 0, sizeof(GenPair) * npair);
+  auto CX = [&](int ps, int m) { return cx + ((size_t)ps * 2 + m) * n2; };
+  auto XC = [&](int ps, int m) { return xc + ((size_t)ps * 2 + m) * n2; };
+  FusedPlan plan;
   for (int p = 0; p < npair; ++p) {
     if (!resident(p)) continue;
     const int psa = 2 * p, psb = 2 * p + 1;
-    auto CX = [&](int ps, int m) { return cx + ((size_t)ps * 2 + m) * n2; };
-    auto XC = [&](int ps, int m) { return xc + ((size_t)ps * 2 + m) * n2; };
     const double* tr_a = &traces[psa * 5];
     const double* tr_b = &traces[psb * 5];
     const double* tr_p = &traces[nps * 5 + p * 8];
@@ -761,14 +916,14 @@ nw_status build_all(nw_ctx* ctx, const std::vector<char>* subset) {
         records_kernel<<<g2, 256>>>(X + (size_t)ps * 2 * n2, Y + (size_t)ps * 2 * n2, Fh + (size_t)ps * 4 * n2,
                                     Vv + (size_t)ps * 8 * n2, Vd + (size_t)ps * 8 * n2, n, recx, recy);
         NW_CUDA(ctx, cudaGetLastError());
-        {
+        if (!fused) {
           nw_status st = transform4(ctx, ctx->d_eri, n, CX(ps, 0), XC(ps, 0), CX(ps, 0), XC(ps, 0), tA, tD, cwp);
           if (st != NW_OK) return st;
           st = transform4(ctx, ctx->d_eri, n, CX(ps, 0), CX(ps, 0), XC(ps, 0), XC(ps, 0), tA, tE, cwp);
           if (st != NW_OK) return st;
+          jas_kernel<<<g4, 256>>>(tD, tE, n, S0 + fo[p].jas[s]);
+          NW_CUDA(ctx, cudaGetLastError());
         }
-        jas_kernel<<<g4, 256>>>(tD, tE, n, S0 + fo[p].jas[s]);
-        NW_CUDA(ctx, cudaGetLastError());
         FastSpin& fs = s ? fp.b : fp.a;
         fs.recx = recx;
         fs.recy = recy;
@@ -777,12 +932,12 @@ nw_status build_all(nw_ctx* ctx, const std::vector<char>* subset) {
         fs.pref = s ? pref_b : pref_a;
         fs.g0 = tr[0] + 0.5 * tr[2];
       }
-      {
+      if (!fused) {
         nw_status st = transform4(ctx, ctx->d_eri, n, CX(psa, 0), XC(psa, 0), CX(psb, 0), XC(psb, 0), tA, tD, cwp);
         if (st != NW_OK) return st;
+        ii_kernel<<<g4, 256>>>(tD, n, S0 + fo[p].ii0);
+        NW_CUDA(ctx, cudaGetLastError());
       }
-      ii_kernel<<<g4, 256>>>(tD, n, S0 + fo[p].ii0);
-      NW_CUDA(ctx, cudaGetLastError());
       fp.ii0 = S0 + fo[p].ii0;
       fp.vab0 = tr_p[0];
     } else {
@@ -815,13 +970,19 @@ nw_status build_all(nw_ctx* ctx, const std::vector<char>* subset) {
             continue;
           }
           const int a = br[sl][0], b = br[sl][1], c = br[sl][2], d = br[sl][3];
+          gs.j[sl] = S0 + g.j[s][sl];
+          if (fused) {
+            // J[a b|c d] = N[cd|ab] - N[ca|db], by the symmetry N'[ab|cd] - N''[ac|bd]
+            plan.add(false, CX(ps, c), XC(ps, d), CX(ps, a), XC(ps, b), S0 + g.j[s][sl]);
+            plan.add(true, CX(ps, c), CX(ps, a), XC(ps, d), XC(ps, b), S0 + g.j[s][sl]);
+            continue;
+          }
           nw_status st = transform4(ctx, ctx->d_eri, n, CX(ps, a), XC(ps, b), CX(ps, c), XC(ps, d), tA, tD, cwp);
           if (st != NW_OK) return st;
           st = transform4(ctx, ctx->d_eri, n, CX(ps, a), CX(ps, c), XC(ps, b), XC(ps, d), tA, tE, cwp);
           if (st != NW_OK) return st;
           jstored_kernel<<<g4, 256>>>(tD, tE, n, S0 + g.j[s][sl]);
           NW_CUDA(ctx, cudaGetLastError());
-          gs.j[sl] = S0 + g.j[s][sl];
         }
         const double* tr = s ? tr_b : tr_a;
         gs.pref = s ? pref_b : pref_a;
@@ -845,11 +1006,15 @@ nw_status build_all(nw_ctx* ctx, const std::vector<char>* subset) {
           gp.ii[a0][az][b0][by] = nullptr;
           continue;
         }
+        gp.ii[a0][az][b0][by] = S0 + g.ii[k];
+        if (fused) {
+          plan.add(false, CX(psa, a0), XC(psa, az), CX(psb, b0), XC(psb, by), S0 + g.ii[k]);
+          continue;
+        }
         nw_status st = transform4(ctx, ctx->d_eri, n, CX(psa, a0), XC(psa, az), CX(psb, b0), XC(psb, by), tA, tD, cwp);
         if (st != NW_OK) return st;
         ii_kernel<<<g4, 256>>>(tD, n, S0 + g.ii[k]);
         NW_CUDA(ctx, cudaGetLastError());
-        gp.ii[a0][az][b0][by] = S0 + g.ii[k];
       }
       for (int i = 0; i < 2; ++i)
         for (int j = 0; j < 2; ++j) {
@@ -857,6 +1022,11 @@ nw_status build_all(nw_ctx* ctx, const std::vector<char>* subset) {
           gp.vba0[j][i] = tr_p[4 + j * 2 + i];
         }
     }
+  }
+
+  if (fused) {
+    const nw_status st = run_fused(ctx, plan, n, nref, resident, generic, fo, CX, XC, S0, tA, tensors);
+    if (st != NW_OK) return st;
   }
 
   // ---------------- tables ----------------

@@ -61,6 +61,7 @@ struct nw_ctx {
   double* d_s = nullptr;
   double* d_h = nullptr;
   double* d_eri = nullptr;
+  int eri_symmetric = -1;   // d_eri has the permutation symmetry of real orbitals (-1: not checked yet)
   double* d_chol = nullptr; // naux x nao x nao Cholesky vectors (nw_ctx_create_cholesky), else null
   int naux = 0;
   int transform = NW_TRANSFORM_FP64;  // four-index transform of the build (nw_set_transform)
@@ -73,6 +74,7 @@ struct nw_ctx {
   size_t slab_bytes = 0;
   size_t slab_capacity = 0;        // bytes allocated at d_slab (>= slab_bytes)
   nw::DevBuf build_work;           // workspace of the build, kept for rebuilds
+  nw::DevBuf build_tasks;          // task tables of the fused transforms
   nw::FastPair* d_fast = nullptr;
   nw::GenPair* d_gen = nullptr;
   int32_t* d_order = nullptr;
@@ -201,6 +203,31 @@ cudaError_t split_product_pqrs(cudaStream_t st, int mode, int slices, const doub
                                double* out, void* scratch, size_t scratch_bytes, uint32_t* err);
 // [p][q][r][s] -> [p][r][q][s] of an n^4 tensor (build.cu).
 cudaError_t swap_qr(cudaStream_t st, const double* src, int n, double* dst);
+
+// Fused half transforms of the four-index tensors (transform.cu), for n <= kTwoSidedMax and a Coulomb
+// tensor with the permutation symmetry of real orbitals.
+constexpr int kTwoSidedMax = 64;
+enum TransformMode { kStore = 0, kSubtract = 1 };
+struct TransformTask {
+  const double* in;   // first half: the Coulomb tensor; second half: H
+  const double* a;    // A (n x n), rows of the result
+  const double* b;    // B (n x n), columns of the result
+  double* out;        // first half: H[pq][u]; second half: N[pq][rs], or J order for kSubtract
+  int mode;           // TransformMode of a second half
+  int pad;
+};
+struct MirrorTask {
+  const double* in;
+  double* out;
+  int o1, o2;         // occupied orbitals of the first and second index pair's spin
+};
+// Leading dimension (even) of H[pq][u], u < n (n + 1) / 2.
+inline size_t packed_ld(int n) { return ((size_t)n * (n + 1) / 2 + 1) / 2 * 2; }
+cudaError_t two_sided(cudaStream_t st, bool half, const TransformTask* tasks, int ntask, int n);
+cudaError_t antisymmetrise(cudaStream_t st, double* const* tensors, int count, int n);
+cudaError_t mirror_tensors(cudaStream_t st, const MirrorTask* tasks, int count, int n);
+// Largest |E| and largest violation of the permutation symmetry (scratch2: two doubles on the device).
+cudaError_t eri_symmetry(cudaStream_t st, const double* eri, int n, double* scratch2, double* big, double* off);
 
 // Build (build.cu).
 // Build of the intermediates of every ordered reference pair, or of the pairs flagged in
