@@ -9,24 +9,31 @@
 // A^{QP}[i][j] = det(C_Q[:, occ(i)]^T S_AO C_P[:, occ(j)]) over the ascending occupied columns of
 // the two alpha strings (B the same for beta), r = the record's phase times the canonical
 // excitation phase of its holes and particles (1 for canonically phased records), so S x is two
-// contractions per ordered parent pair (the B-first order of apply_overlap_sparse,
-// src/noci/factorise/overlap.rs:434-498, 1276-1360):
-//   stage 1  U^{QP}[a][bbar] = sum_{Omega in P, a_Omega = a} r_Omega x_Omega B^{QP}[bbar][b_Omega]
-//   stage 2  y_w += r_w sum_{P != Q} sum_a A^{QP}[a_w][a] U^{QP}[a][b_w]
-// Determinants of one parent are orthonormal, so the same-parent block adds the sources with
-// the same (a, b) pair (the determinant itself in a basis without duplicates).  Per ordered pair
-// the work is nnz(x_P) nb_Q + ndet_Q na_P multiply-adds instead of ndet_Q ndet_P overlaps.
+// contractions per ordered parent pair (apply_overlap_sparse, src/noci/factorise/overlap.rs:434-498,
+// 1276-1360).  With X the sources of P as a matrix over (a, b), the sources are split X = X1 + X2:
+//   stage 1  U[a][bbar] = sum_b X1[a][b] B^{QP}[bbar][b]   for the rows R of X1 (b first)
+//            W[abar][b] = sum_a A^{QP}[abar][a] X2[a][b]   for the columns C of X2 (a first)
+//   stage 2  y_w += r_w sum_P { sum_{a in R} A[a_w][a] U[a][b_w] + sum_{b in C} W[a_w][b] B[b_w][b] }
+// A source goes to X1 when its row is at least as long as its column, so that R and C are the few long
+// rows and columns that cover the sources: for a singles-and-doubles space R is the parent's own alpha
+// string and its singles and C the parent's own beta string, 146 terms a target instead of the 3925
+// alpha strings (n = 40, 4 + 4 electrons), and U and W are 30 MB instead of 740.  All sources by rows
+// or all by columns is taken where that costs less.  Determinants of one parent are orthonormal, so the
+// same-parent block adds the sources with the same (a, b) pair (the determinant itself in a basis
+// without duplicates).
 //
-// Layout: the determinants sorted by (parent, alpha component, beta component); stage 1 takes
-// the sorted sources of each alpha component in chunks of at most 32 (a long row, such as the
-// parent's own alpha string with every beta string, is spread over many blocks that add into its
-// U row) with 256 target beta components per block, reading rows of B^{QP} stored source-major
-// (coalesced over bbar) with four independent loads in flight per thread; stage 2 is one thread
-// per target in sorted order, reading A^{QP} stored source-major too, so for each source string a
-// the lanes of a warp read equal or neighbouring a_w of A and b_w of U (broadcast or coalesced),
-// with the (P, a) sum split into segments whose partial sums a finishing kernel adds in a fixed
-// order.  No allocation and no host synchronisation per apply,
-// so the QMC report block keeps it inside its CUDA graph.
+// Layout: A^{QP} and B^{QP} are stored source-major (row a or b, contiguous over the target's strings,
+// rows padded to an even length), so both stage-1 products read table rows coalesced.  Rows of X1
+// (columns of X2) with mostly the same entries form dense tiles of kOvlTile rows whose sources are
+// staged in shared memory: one 16-byte load of a table row feeds 2 kOvlTile multiply-adds.  The
+// other rows go one by one in chunks of at most kOvlChunk sources, chunks of a long row adding into it
+// atomically.  Stage 2 is one thread per (target, quarter of the terms) in sorted (a, b) order, so
+// a warp reads equal or neighbouring a_w and b_w.  No allocation and no host synchronisation per
+// apply, so the QMC report block keeps it inside its CUDA graph.
+//
+// Bound: HBM, every factor table read once (n = 40, 4 + 4 electrons, 3 references: 1.48 GB, 226 us at the
+// copy bandwidth).  Measured there (B200): 1326 -> 390 us an apply against all sources by rows (stage 1
+// 323 us for all parents, stage 2 52 us; before, 172 and 255 us for each of the three target parents).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -42,29 +49,51 @@
 
 namespace nw {
 
-// Stage 1 works on chunks of at most kOvlChunk sources of one row (a source alpha component a of
-// P for target parent Q): U^{QP}[a][.] is stored by the row's only chunk, or added atomically by
-// each chunk of a longer row (whose U row is cleared first).  A block takes a group of consecutive
-// chunks of one source parent (at most kOvlGroup sources), staged in shared memory.
+// Stage 1, rows one by one: a chunk is a run of sources of one row of X1 (or column of X2); `out` is
+// stored by the row's only chunk, or added into atomically by each chunk of a longer row (cleared first).
+// A block takes a group of consecutive chunks of one table (at most kOvlGroup sources).
 struct OvlChunk {
-  uint64_t bt;    // B^{QP} (source-major, nb_P x nb_Q) in the factor buffer
-  uint64_t urow;  // row a of U^{QP} in the work buffer
-  uint32_t t0, t1;  // sorted source positions
+  uint64_t tab;     // table (source-major) in the factor buffer
+  uint64_t out;     // row of U or W in the work buffer
+  uint32_t k0, k1;  // source list positions
   uint32_t atomic;  // the row has several chunks
   uint32_t pad;
 };
 struct OvlGroup {
   uint32_t c0, c1;  // chunks
-  uint32_t t0, t1;  // their sources
+  uint32_t k0, k1;  // their sources
+  uint32_t ld;      // row length of the table and of the output
+};
+// Stage 1, dense tiles: nrow consecutive output rows over nk common table rows.
+struct OvlTile {
+  uint64_t tab, out;
+  uint64_t x0;      // kOvlTile source entries per table row (the last entry + 1: none)
+  uint32_t k0, nk;  // table rows
+  uint32_t nrow, ld;
+  uint32_t atomic, pad;
+};
+// One source of a row: table row and position among the distinct (parent, a, b) entries.
+struct OvlSource {
+  uint32_t row, entry;
+};
+// Terms of one ordered parent pair in stage 2.
+struct OvlPair {
+  uint64_t a_tab, b_tab;  // factor tables
+  uint64_t u, w;          // first rows of U and W
+  uint32_t r0, nr;        // rows R of the source parent (positions in the row list)
+  uint32_t c0, nc;        // columns C
 };
 
 namespace {
 
 constexpr int kOvlMaxOcc = 16;    // occupied orbitals per spin of the factor kernel
 constexpr int kOvlThreads = 256;
-constexpr uint64_t kOvlThreadTarget = 148ull * 2048 * 4;  // stage-2 threads to aim for (segments): 4 waves
-constexpr uint32_t kOvlChunk = 32;   // sources per stage-1 chunk
-constexpr uint32_t kOvlGroup = 64;   // sources per stage-1 block
+constexpr uint32_t kOvlChunk = 64;    // sources per stage-1 chunk
+constexpr uint32_t kOvlGroup = 64;    // sources per stage-1 block
+constexpr uint32_t kOvlTile = 16;     // rows of a dense stage-1 tile
+constexpr uint32_t kOvlTileK = 160;   // table rows of a dense tile held at once (20 KB of sources)
+constexpr uint32_t kOvlTargets = 64;  // targets of a stage-2 block (kOvlThreads / kOvlTargets term segments)
+constexpr uint64_t kOvlWork = 1ull << 27;  // doubles of U and W per batch of target parents (1 GB)
 
 // One entry of a single-spin factor table per thread; MAXO bounds nocc (the LU scratch lives in
 // the thread's stack frame, MAXO^2 doubles).
@@ -89,47 +118,89 @@ __global__ void __launch_bounds__(kOvlThreads) ovl_factor_kernel(const double* _
   }
 }
 
-__global__ void __launch_bounds__(kOvlThreads) ovl_gather_kernel(uint64_t ndet, const uint32_t* __restrict__ ord_det,
+// xs[e] = sum of r x over the determinants of distinct entry e (xs[nent] = 0 stands for no source), and
+// zeros in the output rows that several chunks add into.
+__global__ void __launch_bounds__(kOvlThreads) ovl_gather_kernel(uint64_t nent, const uint32_t* __restrict__ first,
+                                                                  const uint32_t* __restrict__ ord_det,
                                                                   const double* __restrict__ ord_r,
                                                                   const double* __restrict__ x,
                                                                   double* __restrict__ xs) {
-  for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < ndet; t += (uint64_t)gridDim.x * blockDim.x)
-    xs[t] = ord_r[t] * x[ord_det[t]];
+  for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e <= nent; e += (uint64_t)gridDim.x * blockDim.x) {
+    double v = 0.0;
+    if (e < nent)
+      for (uint32_t t = first[e]; t < first[e + 1]; ++t) v += ord_r[t] * x[ord_det[t]];
+    xs[e] = v;
+  }
 }
 
-// Clears the U rows that several chunks add into (blockIdx.x = row, blockIdx.y = 256 columns).
-__global__ void __launch_bounds__(kOvlThreads) ovl_zero_kernel(const uint64_t* __restrict__ urows, uint32_t ldb,
+__global__ void __launch_bounds__(kOvlThreads) ovl_zero_kernel(const ulonglong2* __restrict__ rows,
                                                                 double* __restrict__ u) {
-  const uint32_t b = blockIdx.y * blockDim.x + threadIdx.x;
-  if (b < ldb) u[urows[blockIdx.x] + b] = 0.0;
+  const ulonglong2 r = rows[blockIdx.x];  // offset, length
+  for (uint64_t i = threadIdx.x; i < r.y; i += blockDim.x) u[r.x + i] = 0.0;
 }
 
-// U^{QP}[a][bbar] for the chunks of one group (blockIdx.x) and 512 target beta components
-// (blockIdx.y), two neighbouring columns per thread (16-byte loads of rows of B^{QP} padded to an
-// even length ldb): every thread sums its columns over the group's staged sources; the loads of
-// one chunk are independent (four in flight per step).
-__global__ void __launch_bounds__(kOvlThreads) ovl_stage1_kernel(const OvlGroup* __restrict__ groups,
-                                                                  const OvlChunk* __restrict__ chunks,
-                                                                  const uint32_t* __restrict__ ord_b,
-                                                                  const double* __restrict__ xs,
-                                                                  const double* __restrict__ fac, uint32_t ldb,
-                                                                  double* __restrict__ u) {
-  __shared__ double sx[kOvlGroup];
-  __shared__ uint32_t sb[kOvlGroup];
-  const OvlGroup g = groups[blockIdx.x];
-  for (uint32_t i = threadIdx.x; i < g.t1 - g.t0; i += blockDim.x) {
-    sx[i] = xs[g.t0 + i];
-    sb[i] = ord_b[g.t0 + i];
+// Stage 1: blockIdx.x < ntile takes a dense tile (bound by FP64 FMA), the others a group of chunks (bound by
+// reading the table); both in one launch, so the tiles' arithmetic runs beside the others' loads.
+// blockIdx.y takes 512 columns, two neighbouring ones per thread.
+__global__ void __launch_bounds__(kOvlThreads, 3)
+    ovl_stage1_kernel(const OvlTile* __restrict__ tiles, uint32_t ntile, const OvlGroup* __restrict__ groups,
+                      const OvlChunk* __restrict__ chunks, const OvlSource* __restrict__ src,
+                      const uint32_t* __restrict__ trow, const uint32_t* __restrict__ tent,
+                      const double* __restrict__ xs, const double* __restrict__ fac, double* __restrict__ u) {
+  __shared__ __align__(16) double sx[kOvlTileK * kOvlTile];
+  __shared__ uint32_t sb[kOvlTileK];
+  const uint32_t col = 2 * (blockIdx.y * blockDim.x + threadIdx.x);
+  if (blockIdx.x < ntile) {
+    const OvlTile t = tiles[blockIdx.x];
+    if (2 * blockIdx.y * blockDim.x >= t.ld) return;
+    double2 acc[kOvlTile];
+#pragma unroll
+    for (uint32_t i = 0; i < kOvlTile; ++i) acc[i] = make_double2(0.0, 0.0);
+    for (uint32_t kb = 0; kb < t.nk; kb += kOvlTileK) {
+      const uint32_t nk = min(kOvlTileK, t.nk - kb);
+      __syncthreads();
+      for (uint32_t i = threadIdx.x; i < nk * kOvlTile; i += blockDim.x) sx[i] = xs[tent[t.x0 + kb * kOvlTile + i]];
+      for (uint32_t i = threadIdx.x; i < nk; i += blockDim.x) sb[i] = trow[t.k0 + kb + i];
+      __syncthreads();
+      if (col < t.ld) {
+        const double* tab = fac + t.tab + col;
+        double2 next = __ldg(reinterpret_cast<const double2*>(tab + (uint64_t)sb[0] * t.ld));
+#pragma unroll 2
+        for (uint32_t k = 0; k < nk; ++k) {
+          const double2 b = next;
+          if (k + 1 < nk) next = __ldg(reinterpret_cast<const double2*>(tab + (uint64_t)sb[k + 1] * t.ld));
+          const double2* xr = reinterpret_cast<const double2*>(sx + k * kOvlTile);
+#pragma unroll
+          for (uint32_t i = 0; i < kOvlTile / 2; ++i) {
+            const double2 xv = xr[i];
+            acc[2 * i].x = fma(xv.x, b.x, acc[2 * i].x);
+            acc[2 * i].y = fma(xv.x, b.y, acc[2 * i].y);
+            acc[2 * i + 1].x = fma(xv.y, b.x, acc[2 * i + 1].x);
+            acc[2 * i + 1].y = fma(xv.y, b.y, acc[2 * i + 1].y);
+          }
+        }
+      }
+    }
+    if (col >= t.ld) return;
+#pragma unroll
+    for (uint32_t i = 0; i < kOvlTile; ++i)
+      if (i < t.nrow) *reinterpret_cast<double2*>(u + t.out + (uint64_t)i * t.ld + col) = acc[i];
+    return;
+  }
+  const OvlGroup g = groups[blockIdx.x - ntile];
+  for (uint32_t i = threadIdx.x; i < g.k1 - g.k0; i += blockDim.x) {
+    const OvlSource s = src[g.k0 + i];
+    sx[i] = xs[s.entry];
+    sb[i] = s.row;
   }
   __syncthreads();
-  const uint32_t col = 2 * (blockIdx.y * blockDim.x + threadIdx.x);
-  if (col >= ldb) return;
+  if (col >= g.ld) return;
   for (uint32_t c = g.c0; c < g.c1; ++c) {
     const OvlChunk ch = chunks[c];
-    const double* bt = fac + ch.bt + col;
-    auto row = [&](uint32_t k) { return __ldg(reinterpret_cast<const double2*>(bt + (uint64_t)sb[k] * ldb)); };
-    const uint32_t k1 = ch.t1 - g.t0;
-    uint32_t k = ch.t0 - g.t0;
+    const double* bt = fac + ch.tab + col;
+    auto row = [&](uint32_t k) { return __ldg(reinterpret_cast<const double2*>(bt + (uint64_t)sb[k] * g.ld)); };
+    const uint32_t k1 = ch.k1 - g.k0;
+    uint32_t k = ch.k0 - g.k0;
     double2 a0 = make_double2(0.0, 0.0), a1 = a0, a2 = a0, a3 = a0;
     for (; k + 4 <= k1; k += 4) {
       const double2 b0 = row(k), b1 = row(k + 1), b2 = row(k + 2), b3 = row(k + 3);
@@ -148,7 +219,7 @@ __global__ void __launch_bounds__(kOvlThreads) ovl_stage1_kernel(const OvlGroup*
       a0.y += sx[k] * b0.y;
     }
     const double s0 = (a0.x + a1.x) + (a2.x + a3.x), s1 = (a0.y + a1.y) + (a2.y + a3.y);
-    double* dst = u + ch.urow + col;
+    double* dst = u + ch.out + col;
     if (ch.atomic) {
       atomicAdd(dst, s0);
       atomicAdd(dst + 1, s1);
@@ -158,71 +229,72 @@ __global__ void __launch_bounds__(kOvlThreads) ovl_stage1_kernel(const OvlGroup*
   }
 }
 
-// Partial sums over segment blockIdx.y of the (P, a) index of every target t in [t0, t1) of
-// parent q: part[seg][t] = sum A^{qP}[a_t][a] U^{qP}[a][b_t].  A is stored source-major
-// (row a holds the na_q targets' strings), so for a fixed a the lanes of a warp read
-// neighbouring or equal a_t (one run of a string's targets, or the doubly excited strings one
-// target each) as they read neighbouring or equal b_t of U: both loads coalesce or broadcast.
-__global__ void __launch_bounds__(kOvlThreads) ovl_stage2_kernel(int q, int nref, uint64_t t0, uint64_t t1,
-                                                                  uint64_t seglen, const uint32_t* __restrict__ ord_a,
-                                                                  const uint32_t* __restrict__ ord_b,
-                                                                  const uint32_t* __restrict__ na,
-                                                                  const uint64_t* __restrict__ a_off,
-                                                                  const uint64_t* __restrict__ u_off, uint32_t naq,
-                                                                  uint32_t ldb, const double* __restrict__ fac,
-                                                                  const double* __restrict__ u, uint64_t ndet,
-                                                                  double* __restrict__ part) {
-  const uint64_t t = t0 + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (t >= t1) return;
-  const uint64_t k0 = (uint64_t)blockIdx.y * seglen, k1 = k0 + seglen;
-  const uint32_t at = ord_a[t], bq = ord_b[t];
-  double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0, acc3 = 0.0;
-  uint64_t kbase = 0;
-  for (int p = 0; p < nref; ++p) {
-    if (p == q) continue;
-    const uint64_t n = na[p];
-    const uint64_t lo = k0 > kbase ? k0 : kbase;
-    const uint64_t hi = k1 < kbase + n ? k1 : kbase + n;
-    if (lo < hi) {
-      // a = k - kbase runs over [lo - kbase, hi - kbase) of this parent's alpha components
-      const double* acol = fac + a_off[(uint64_t)q * nref + p] + at;
-      const double* ucol = u + u_off[(uint64_t)q * nref + p] + bq;
-      const uint64_t a1 = hi - kbase;
-      uint64_t a = lo - kbase;
-      for (; a + 4 <= a1; a += 4) {
-        const double u0 = __ldg(ucol + a * ldb), u1 = __ldg(ucol + (a + 1) * ldb);
-        const double u2 = __ldg(ucol + (a + 2) * ldb), u3 = __ldg(ucol + (a + 3) * ldb);
-        acc0 += __ldg(acol + a * naq) * u0;
-        acc1 += __ldg(acol + (a + 1) * naq) * u1;
-        acc2 += __ldg(acol + (a + 2) * naq) * u2;
-        acc3 += __ldg(acol + (a + 3) * naq) * u3;
+// y_t += r_t (sum of the stage-2 terms + same-parent sources) for kOvlTargets sorted targets of one
+// parent per block; each of the kOvlThreads / kOvlTargets thread rows sums one segment of the terms
+// (all P != Q, R then C), added in a fixed order through shared memory.
+__global__ void __launch_bounds__(kOvlThreads)
+    ovl_stage2_kernel(int q0, int nref, const uint32_t* __restrict__ blk, const uint64_t* __restrict__ pstart,
+                      const OvlPair* __restrict__ pairs, const uint32_t* __restrict__ rlist,
+                      const uint32_t* __restrict__ clist, const uint32_t* __restrict__ lda,
+                      const uint32_t* __restrict__ ldb, const uint32_t* __restrict__ ord_det,
+                      const uint32_t* __restrict__ ord_a, const uint32_t* __restrict__ ord_b,
+                      const uint32_t* __restrict__ ord_e, const double* __restrict__ ord_r,
+                      const double* __restrict__ xs, const double* __restrict__ fac, const double* __restrict__ u,
+                      double* __restrict__ y) {
+  constexpr int kSeg = kOvlThreads / kOvlTargets;
+  __shared__ double part[kSeg][kOvlTargets];
+  int q = q0;
+  const uint32_t b0 = blk[q0] + blockIdx.x;
+  while (b0 >= blk[q + 1]) ++q;
+  const int tl = threadIdx.x % kOvlTargets, seg = threadIdx.x / kOvlTargets;
+  const uint64_t t = pstart[q] + (uint64_t)(b0 - blk[q]) * kOvlTargets + tl;
+  const bool live = t < pstart[q + 1];
+  double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+  if (live) {
+    const uint32_t at = ord_a[t], bt = ord_b[t];
+    const uint64_t la = lda[q], lb = ldb[q];
+    for (int p = 0; p < nref; ++p) {
+      if (p == q) continue;
+      const OvlPair pr = pairs[(uint64_t)q * nref + p];
+      {
+        const uint32_t k1 = (uint32_t)((uint64_t)pr.nr * (seg + 1) / kSeg);
+        uint32_t k = (uint32_t)((uint64_t)pr.nr * seg / kSeg);
+        const uint32_t* rl = rlist + pr.r0;
+        const double* av = fac + pr.a_tab + at;
+        const double* uv = u + pr.u + bt;
+        for (; k + 4 <= k1; k += 4) {
+          const uint64_t r0 = __ldg(rl + k), r1 = __ldg(rl + k + 1), r2 = __ldg(rl + k + 2), r3 = __ldg(rl + k + 3);
+          a0 += __ldg(av + r0 * la) * uv[k * lb];
+          a1 += __ldg(av + r1 * la) * uv[(k + 1) * lb];
+          a2 += __ldg(av + r2 * la) * uv[(k + 2) * lb];
+          a3 += __ldg(av + r3 * la) * uv[(k + 3) * lb];
+        }
+        for (; k < k1; ++k) a0 += __ldg(av + (uint64_t)__ldg(rl + k) * la) * uv[k * lb];
       }
-      for (; a < a1; ++a) acc0 += __ldg(acol + a * naq) * __ldg(ucol + a * ldb);
+      {
+        const uint32_t k1 = (uint32_t)((uint64_t)pr.nc * (seg + 1) / kSeg);
+        uint32_t k = (uint32_t)((uint64_t)pr.nc * seg / kSeg);
+        const uint32_t* cl = clist + pr.c0;
+        const double* bv = fac + pr.b_tab + bt;
+        const double* wv = u + pr.w + at;
+        for (; k + 4 <= k1; k += 4) {
+          const uint64_t c0 = __ldg(cl + k), c1 = __ldg(cl + k + 1), c2 = __ldg(cl + k + 2), c3 = __ldg(cl + k + 3);
+          a0 += __ldg(bv + c0 * lb) * wv[k * la];
+          a1 += __ldg(bv + c1 * lb) * wv[(k + 1) * la];
+          a2 += __ldg(bv + c2 * lb) * wv[(k + 2) * la];
+          a3 += __ldg(bv + c3 * lb) * wv[(k + 3) * la];
+        }
+        for (; k < k1; ++k) a0 += __ldg(bv + (uint64_t)__ldg(cl + k) * lb) * wv[k * la];
+      }
     }
-    kbase += n;
   }
-  part[(uint64_t)blockIdx.y * ndet + t] = (acc0 + acc1) + (acc2 + acc3);
-}
-
-__global__ void __launch_bounds__(kOvlThreads) ovl_finish_kernel(uint64_t ndet, int nseg, int cross,
-                                                                  const uint32_t* __restrict__ ord_det,
-                                                                  const double* __restrict__ ord_r,
-                                                                  const uint32_t* __restrict__ run_lo,
-                                                                  const uint32_t* __restrict__ run_hi,
-                                                                  const double* __restrict__ xs,
-                                                                  const double* __restrict__ part,
-                                                                  double* __restrict__ y) {
-  for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < ndet; t += (uint64_t)gridDim.x * blockDim.x) {
+  part[seg][tl] = (a0 + a1) + (a2 + a3);
+  __syncthreads();
+  if (seg == 0 && live) {
     double v = 0.0;
-    if (cross)
-      for (int s = 0; s < nseg; ++s) v += part[(uint64_t)s * ndet + t];
-    double same = 0.0;
-    if (run_lo) {
-      for (uint32_t k = run_lo[t]; k < run_hi[t]; ++k) same += xs[k];
-    } else {
-      same = xs[t];
-    }
-    y[ord_det[t]] += ord_r[t] * (v + same);
+#pragma unroll
+    for (int s = 0; s < kSeg; ++s) v += part[s][tl];
+    y[ord_det[t]] += ord_r[t] * (v + xs[ord_e[t]]);
   }
 }
 
@@ -268,33 +340,109 @@ SpinKey spin_key(int rank, const uint8_t* idx) {
 }  // namespace
 
 struct OverlapPlan {
+  // Target parents [q0, q1) whose U and W fit the work buffer together, with their stage-1 work.
+  struct Batch {
+    int q0, q1;
+    uint64_t tile0, ntile, group0, ngroup, zero0, nzero;
+    uint32_t ldmax;
+    uint32_t nblk;  // stage-2 blocks
+  };
   int nref = 0, oa = 0, ob = 0;
-  uint64_t ndet = 0;
-  int nseg = 1;
+  uint64_t ndet = 0, nent = 0;
   std::vector<uint32_t> na, nb;
-  std::vector<uint32_t> ldb;            // beta strings per parent rounded up to even: row stride of B and U
+  std::vector<uint32_t> lda, ldb;       // alpha / beta strings per parent rounded up to even: table row lengths
   std::vector<uint64_t> pstart;         // per parent: first sorted position (nref + 1)
-  std::vector<uint64_t> ngroups, groups_off;  // per target parent: stage-1 groups
-  std::vector<uint64_t> nzero, zero_off;      // per target parent: U rows cleared before stage 1
-  std::vector<uint64_t> seglen;         // per target parent
+  std::vector<Batch> batches;
   void* mem = nullptr;
   uint32_t* ord_det = nullptr;
   uint32_t* ord_a = nullptr;
   uint32_t* ord_b = nullptr;
+  uint32_t* ord_e = nullptr;
   double* ord_r = nullptr;
-  uint32_t* run_lo = nullptr;  // null when every (parent, a, b) is a single determinant
-  uint32_t* run_hi = nullptr;
+  uint32_t* first = nullptr;            // first sorted position of each distinct entry (nent + 1)
+  OvlTile* tiles = nullptr;
   OvlGroup* groups = nullptr;
   OvlChunk* chunks = nullptr;
-  uint64_t* zero_rows = nullptr;
-  uint64_t* d_a_off = nullptr;
-  uint64_t* d_u_off = nullptr;
-  uint32_t* d_na = nullptr;
+  OvlSource* src = nullptr;
+  uint32_t* trow = nullptr;
+  uint32_t* tent = nullptr;
+  ulonglong2* zero_rows = nullptr;
+  OvlPair* pairs = nullptr;
+  uint32_t* rlist = nullptr;
+  uint32_t* clist = nullptr;
+  uint32_t* d_lda = nullptr;
+  uint32_t* d_ldb = nullptr;
+  uint32_t* d_blk = nullptr;
+  uint64_t* d_pstart = nullptr;
   double* fac = nullptr;
   double* u = nullptr;
   double* xs = nullptr;
-  double* part = nullptr;
 };
+
+namespace {
+
+// The sources of one parent by rows (or columns): for each line its id and its (table row, entry) list.
+struct Lines {
+  std::vector<uint32_t> id;
+  std::vector<std::vector<OvlSource>> src;
+};
+
+// Split of one parent's distinct entries into lines by rows (R) and by columns (C), see the header.  `rows` and
+// `cols` count each alpha and beta string's entries; targets, nb and na are the other parents' averages.
+void split_sources(const std::vector<uint32_t>& ea, const std::vector<uint32_t>& eb, uint32_t na, uint32_t nb,
+                   uint64_t e0, double targets, double tna, double tnb, Lines* R, Lines* C) {
+  const size_t ne = ea.size();
+  std::vector<uint32_t> rows(na, 0), cols(nb, 0);
+  for (size_t e = 0; e < ne; ++e) {
+    ++rows[ea[e]];
+    ++cols[eb[e]];
+  }
+  auto by_row = [&](int mode, size_t e) { return mode == 0 ? rows[ea[e]] >= cols[eb[e]] : mode == 1; };
+  int best = 0;
+  double best_cost = 0.0;
+  for (int mode = 0; mode < 3; ++mode) {  // the rule, all by rows, all by columns
+    std::vector<char> r(na, 0), c(nb, 0);
+    double cost = 0.0;
+    for (size_t e = 0; e < ne; ++e) {
+      if (by_row(mode, e)) {
+        r[ea[e]] = 1;
+        cost += tnb;
+      } else {
+        c[eb[e]] = 1;
+        cost += tna;
+      }
+    }
+    for (char k : r) cost += k ? targets : 0.0;
+    for (char k : c) cost += k ? targets : 0.0;
+    if (mode == 0 || cost < best_cost) {
+      best = mode;
+      best_cost = cost;
+    }
+  }
+  std::vector<std::vector<OvlSource>> lr(na), lc(nb);
+  for (size_t e = 0; e < ne; ++e) {
+    if (by_row(best, e))
+      lr[ea[e]].push_back(OvlSource{eb[e], (uint32_t)(e0 + e)});
+    else
+      lc[eb[e]].push_back(OvlSource{ea[e], (uint32_t)(e0 + e)});
+  }
+  auto collect = [](std::vector<std::vector<OvlSource>>& l, Lines* out) {
+    std::vector<uint32_t> id;
+    for (uint32_t i = 0; i < l.size(); ++i)
+      if (!l[i].empty()) id.push_back(i);
+    // lines of equal length next to each other, so that lines with the same entries share a tile
+    std::stable_sort(id.begin(), id.end(), [&](uint32_t x, uint32_t y) { return l[x].size() > l[y].size(); });
+    for (uint32_t i : id) {
+      out->id.push_back(i);
+      std::sort(l[i].begin(), l[i].end(), [](const OvlSource& x, const OvlSource& y) { return x.row < y.row; });
+      out->src.push_back(std::move(l[i]));
+    }
+  };
+  collect(lr, R);
+  collect(lc, C);
+}
+
+}  // namespace
 
 void overlap_plan_free(OverlapPlan* pl) {
   if (!pl) return;
@@ -337,11 +485,13 @@ nw_status overlap_plan_get(nw_ctx* ctx, cudaStream_t stream, OverlapPlan** out) 
   }
   pl->na.resize(nref);
   pl->nb.resize(nref);
+  pl->lda.resize(nref);
   pl->ldb.resize(nref);
   std::vector<uint64_t> ca_off(nref + 1, 0), cb_off(nref + 1, 0);
   for (int p = 0; p < nref; ++p) {
     pl->na[p] = (uint32_t)ca[p].size();
     pl->nb[p] = (uint32_t)cb[p].size();
+    pl->lda[p] = (pl->na[p] + 1) & ~1u;
     pl->ldb[p] = (pl->nb[p] + 1) & ~1u;
     ca_off[p + 1] = ca_off[p] + pl->na[p];
     cb_off[p + 1] = cb_off[p] + pl->nb[p];
@@ -373,86 +523,167 @@ nw_status overlap_plan_get(nw_ctx* ctx, cudaStream_t stream, OverlapPlan** out) 
     if (bid[x] != bid[y]) return bid[x] < bid[y];
     return x < y;
   });
-  std::vector<uint32_t> o_a(nd), o_b(nd), run_lo(nd), run_hi(nd);
+  std::vector<uint32_t> o_a(nd), o_b(nd), o_e(nd), first;
   std::vector<double> o_r(nd);
-  std::vector<uint64_t> rowstart(ca_off[nref] + 1, 0);
   pl->pstart.assign(nref + 1, nd);
-  bool dups = false;
+  // distinct (parent, a, b) entries in sorted order
+  std::vector<std::vector<uint32_t>> ea(nref), eb(nref);
+  std::vector<uint64_t> estart(nref + 1, 0);
   for (uint64_t t = 0; t < nd; ++t) {
     const uint32_t d = order[t];
     const uint32_t p = dets[d].parent;
     o_a[t] = aid[d];
     o_b[t] = bid[d];
     o_r[t] = rr[d];
-    if (t == 0 || dets[order[t - 1]].parent != p) pl->pstart[p] = t;
-    if (t == 0 || dets[order[t - 1]].parent != p || aid[order[t - 1]] != aid[d]) rowstart[ca_off[p] + aid[d]] = t;
+    const bool np = t == 0 || dets[order[t - 1]].parent != p;
+    if (np) pl->pstart[p] = t;
+    if (np || o_a[t - 1] != o_a[t] || o_b[t - 1] != o_b[t]) {
+      first.push_back((uint32_t)t);
+      ea[p].push_back(o_a[t]);
+      eb[p].push_back(o_b[t]);
+    }
+    o_e[t] = (uint32_t)first.size() - 1;
   }
-  rowstart[ca_off[nref]] = nd;
+  pl->nent = first.size();
+  first.push_back((uint32_t)nd);
+  for (int p = 0; p < nref; ++p) estart[p + 1] = estart[p] + ea[p].size();
   for (int p = nref - 1; p >= 0; --p)
     if (pl->pstart[p] > pl->pstart[p + 1]) pl->pstart[p] = pl->pstart[p + 1];  // parents without determinants
-  for (uint64_t t = 0; t < nd;) {
-    uint64_t e = t + 1;
-    while (e < nd && dets[order[e]].parent == dets[order[t]].parent && o_a[e] == o_a[t] && o_b[e] == o_b[t]) ++e;
-    if (e - t > 1) dups = true;
-    for (uint64_t k = t; k < e; ++k) {
-      run_lo[k] = (uint32_t)t;
-      run_hi[k] = (uint32_t)e;
-    }
-    t = e;
+  // rows and columns of every source parent
+  std::vector<Lines> R(nref), C(nref);
+  std::vector<uint32_t> rlist, clist, r0(nref), c0(nref);
+  for (int p = 0; p < nref && nref > 1; ++p) {
+    double targets = 0.0, tna = 0.0, tnb = 0.0;
+    for (int q = 0; q < nref; ++q)
+      if (q != p) {
+        targets += (double)(pl->pstart[q + 1] - pl->pstart[q]);
+        tna += pl->na[q];
+        tnb += pl->nb[q];
+      }
+    split_sources(ea[p], eb[p], pl->na[p], pl->nb[p], estart[p], targets, tna, tnb, &R[p], &C[p]);
+    r0[p] = (uint32_t)rlist.size();
+    c0[p] = (uint32_t)clist.size();
+    rlist.insert(rlist.end(), R[p].id.begin(), R[p].id.end());
+    clist.insert(clist.end(), C[p].id.begin(), C[p].id.end());
   }
-  // factor tables, U offsets and stage-1 rows
-  std::vector<uint64_t> a_off((size_t)nref * nref, 0), bt_off((size_t)nref * nref, 0), u_off((size_t)nref * nref, 0);
+  // factor tables, U and W rows and the stage-1 work per batch of target parents
+  std::vector<uint64_t> a_off((size_t)nref * nref, 0), bt_off((size_t)nref * nref, 0);
+  std::vector<OvlPair> pairs((size_t)nref * nref, OvlPair{});
   uint64_t nfac = 0, nu = 0;
+  std::vector<OvlTile> tiles;
   std::vector<OvlGroup> groups;
   std::vector<OvlChunk> chunks;
-  std::vector<uint64_t> zero_rows;
-  pl->ngroups.assign(nref, 0);
-  pl->groups_off.assign(nref, 0);
-  pl->nzero.assign(nref, 0);
-  pl->zero_off.assign(nref, 0);
-  pl->seglen.assign(nref, 1);
-  uint64_t max_targets = 1;
-  for (int q = 0; q < nref; ++q) max_targets = std::max<uint64_t>(max_targets, pl->pstart[q + 1] - pl->pstart[q]);
-  pl->nseg = (int)std::max<uint64_t>(1, std::min<uint64_t>(64, (kOvlThreadTarget + max_targets - 1) / max_targets));
-  for (int q = 0; q < nref; ++q) {
-    uint64_t uq = 0, kq = 0;
-    pl->groups_off[q] = groups.size();
-    pl->zero_off[q] = zero_rows.size();
-    for (int p = 0; p < nref; ++p) {
-      if (p == q) continue;
-      const size_t i = (size_t)q * nref + p;
-      a_off[i] = nfac;
-      nfac += (uint64_t)pl->na[q] * pl->na[p];
-      nfac = (nfac + 1) & ~1ull;  // 16-byte aligned rows of B
-      bt_off[i] = nfac;
-      nfac += (uint64_t)pl->nb[p] * pl->ldb[q];
-      u_off[i] = uq;
-      // chunks of the rows of P in sorted order, grouped (a group never spans two parents)
-      bool open = false;
-      for (uint32_t a = 0; a < pl->na[p]; ++a) {
-        const uint64_t r0 = rowstart[ca_off[p] + a], r1 = rowstart[ca_off[p] + a + 1];
-        const uint64_t urow = uq + (uint64_t)a * pl->ldb[q];
-        const bool multi = r1 - r0 > kOvlChunk;
-        if (multi) zero_rows.push_back(urow);
-        for (uint64_t c0 = r0; c0 < r1; c0 += kOvlChunk) {
-          const uint64_t c1 = std::min<uint64_t>(r1, c0 + kOvlChunk);
-          if (!open || c1 - groups.back().t0 > kOvlGroup) {
-            groups.push_back(OvlGroup{(uint32_t)chunks.size(), (uint32_t)chunks.size(), (uint32_t)c0, (uint32_t)c0});
-            open = true;
+  std::vector<OvlSource> src;
+  std::vector<uint32_t> trow, tent, blk(nref + 1, 0);
+  std::vector<ulonglong2> zero_rows;
+  for (int q = 0; q < nref; ++q)
+    blk[q + 1] = blk[q] + (uint32_t)((pl->pstart[q + 1] - pl->pstart[q] + kOvlTargets - 1) / kOvlTargets);
+  // the lists of one source parent's lines are shared by all its targets: tile and chunk shapes per line set
+  struct Shape {
+    bool tile;
+    uint32_t l0, nl;     // lines
+    uint32_t k0, nk;     // tile: table rows; line: sources in `src`
+    uint64_t x0;
+  };
+  auto shapes_of = [&](const Lines& L) {
+    std::vector<Shape> out;
+    for (uint32_t l = 0; l < L.id.size();) {
+      // a tile where the lines share their entries: at most 1.5 times the work of the lines one by one
+      const uint32_t nl = std::min<uint32_t>(kOvlTile, (uint32_t)L.id.size() - l);
+      std::vector<uint32_t> rows;
+      uint64_t nnz = 0;
+      for (uint32_t i = 0; i < nl; ++i)
+        for (const OvlSource& s : L.src[l + i]) {
+          rows.push_back(s.row);
+          ++nnz;
+        }
+      std::sort(rows.begin(), rows.end());
+      rows.erase(std::unique(rows.begin(), rows.end()), rows.end());
+      if (nl >= 4 && 2 * rows.size() * nl <= 3 * nnz) {
+        const Shape sh{true, l, nl, (uint32_t)trow.size(), (uint32_t)rows.size(), tent.size()};
+        trow.insert(trow.end(), rows.begin(), rows.end());
+        tent.resize(sh.x0 + rows.size() * kOvlTile, (uint32_t)pl->nent);
+        for (uint32_t i = 0; i < nl; ++i)
+          for (const OvlSource& s : L.src[l + i]) {
+            const size_t k = std::lower_bound(rows.begin(), rows.end(), s.row) - rows.begin();
+            tent[sh.x0 + k * kOvlTile + i] = s.entry;
           }
-          chunks.push_back(OvlChunk{bt_off[i], urow, (uint32_t)c0, (uint32_t)c1, multi ? 1u : 0u, 0u});
-          groups.back().c1 = (uint32_t)chunks.size();
-          groups.back().t1 = (uint32_t)c1;
+        out.push_back(sh);
+        l += nl;
+      } else {
+        out.push_back(Shape{false, l, 1, (uint32_t)src.size(), (uint32_t)L.src[l].size(), 0});
+        src.insert(src.end(), L.src[l].begin(), L.src[l].end());
+        ++l;
+      }
+    }
+    return out;
+  };
+  std::vector<std::vector<Shape>> rshape(nref), cshape(nref);
+  for (int p = 0; p < nref; ++p) {
+    rshape[p] = shapes_of(R[p]);
+    cshape[p] = shapes_of(C[p]);
+  }
+  auto work_of = [&](int q) {
+    uint64_t w = 0;
+    for (int p = 0; p < nref; ++p)
+      if (p != q) w += (uint64_t)R[p].id.size() * pl->ldb[q] + (uint64_t)C[p].id.size() * pl->lda[q];
+    return w;
+  };
+  for (int q = 0; q < nref && nref > 1;) {
+    OverlapPlan::Batch bt{q, q, tiles.size(), 0, groups.size(), 0, zero_rows.size(), 0, 2, 0};
+    uint64_t uq = 0;
+    while (bt.q1 < nref && (bt.q1 == bt.q0 || uq + work_of(bt.q1) <= kOvlWork)) {
+      const int qq = bt.q1++;
+      bt.nblk += blk[qq + 1] - blk[qq];
+      if (pl->pstart[qq + 1] == pl->pstart[qq]) continue;
+      bt.ldmax = std::max(bt.ldmax, std::max(pl->lda[qq], pl->ldb[qq]));
+      for (int p = 0; p < nref; ++p) {
+        if (p == qq) continue;
+        const size_t i = (size_t)qq * nref + p;
+        nfac = (nfac + 1) & ~1ull;  // 16-byte aligned table rows
+        a_off[i] = nfac;
+        nfac += (uint64_t)pl->na[p] * pl->lda[qq];
+        bt_off[i] = nfac;
+        nfac += (uint64_t)pl->nb[p] * pl->ldb[qq];
+        OvlPair& pr = pairs[i];
+        pr = OvlPair{a_off[i], bt_off[i], 0, 0, r0[p], (uint32_t)R[p].id.size(), c0[p], (uint32_t)C[p].id.size()};
+        for (int side = 0; side < 2; ++side) {
+          const uint32_t ld = side ? pl->lda[qq] : pl->ldb[qq];
+          const uint64_t tab = side ? a_off[i] : bt_off[i];
+          (side ? pr.w : pr.u) = uq;
+          bool open = false;  // a group never spans two tables
+          for (const Shape& sh : side ? cshape[p] : rshape[p]) {
+            const uint64_t out = uq + (uint64_t)sh.l0 * ld;
+            if (sh.tile) {
+              tiles.push_back(OvlTile{tab, out, sh.x0, sh.k0, sh.nk, sh.nl, ld, 0u, 0u});
+              continue;
+            }
+            const bool multi = sh.nk > kOvlChunk;
+            if (multi) zero_rows.push_back(make_ulonglong2(out, ld));
+            for (uint32_t k = 0; k < sh.nk; k += kOvlChunk) {
+              const uint32_t ka = sh.k0 + k, kb = sh.k0 + std::min(sh.nk, k + kOvlChunk);
+              // a group's sources are consecutive in the list (a tile between two lines does not break that)
+              if (!open || kb - groups.back().k0 > kOvlGroup || ka != groups.back().k1) {
+                groups.push_back(OvlGroup{(uint32_t)chunks.size(), (uint32_t)chunks.size(), ka, ka, ld});
+                open = true;
+              }
+              chunks.push_back(OvlChunk{tab, out, ka, kb, multi ? 1u : 0u, 0u});
+              groups.back().c1 = (uint32_t)chunks.size();
+              groups.back().k1 = kb;
+            }
+          }
+          uq += (uint64_t)(side ? C[p].id.size() : R[p].id.size()) * ld;
         }
       }
-      uq += (uint64_t)pl->na[p] * pl->ldb[q];
-      kq += pl->na[p];
     }
-    pl->ngroups[q] = groups.size() - pl->groups_off[q];
-    pl->nzero[q] = zero_rows.size() - pl->zero_off[q];
-    pl->seglen[q] = std::max<uint64_t>(1, (kq + pl->nseg - 1) / pl->nseg);
+    bt.ntile = tiles.size() - bt.tile0;
+    bt.ngroup = groups.size() - bt.group0;
+    bt.nzero = zero_rows.size() - bt.zero0;
     nu = std::max(nu, uq);
+    pl->batches.push_back(bt);
+    q = bt.q1;
   }
+  if (nref == 1) pl->batches.push_back(OverlapPlan::Batch{0, 1, 0, 0, 0, 0, 0, 0, 2, blk[1]});
   // one allocation: device arrays, factor tables, work buffers and the MO overlaps of the set-up
   const size_t n2 = (size_t)nmo * nmo;
   const size_t nrr = (size_t)nref * nref;
@@ -462,15 +693,22 @@ nw_status overlap_plan_get(nw_ctx* ctx, cudaStream_t stream, OverlapPlan** out) 
     off += (bytes + 255) & ~(size_t)255;
     return at;
   };
-  const size_t o_det = carve(nd * 4), o_a_ = carve(nd * 4), o_b_ = carve(nd * 4), o_r_ = carve(nd * 8);
-  const size_t o_lo = dups ? carve(nd * 4) : 0, o_hi = dups ? carve(nd * 4) : 0;
-  const size_t o_groups = carve(std::max<size_t>(1, groups.size()) * sizeof(OvlGroup));
-  const size_t o_chunks = carve(std::max<size_t>(1, chunks.size()) * sizeof(OvlChunk));
-  const size_t o_zero = carve(std::max<size_t>(1, zero_rows.size()) * 8);
-  const size_t o_aoff = carve(nrr * 8), o_uoff = carve(nrr * 8), o_na = carve(nref * 4);
+  auto some = [](size_t n) { return std::max<size_t>(1, n); };
+  const size_t o_det = carve(nd * 4), o_a_ = carve(nd * 4), o_b_ = carve(nd * 4), o_e_ = carve(nd * 4);
+  const size_t o_r_ = carve(nd * 8), o_first = carve(first.size() * 4);
+  const size_t o_tiles = carve(some(tiles.size()) * sizeof(OvlTile));
+  const size_t o_groups = carve(some(groups.size()) * sizeof(OvlGroup));
+  const size_t o_chunks = carve(some(chunks.size()) * sizeof(OvlChunk));
+  const size_t o_src = carve(some(src.size()) * sizeof(OvlSource));
+  const size_t o_trow = carve(some(trow.size()) * 4), o_tent = carve(some(tent.size()) * 4);
+  const size_t o_zero = carve(some(zero_rows.size()) * sizeof(ulonglong2));
+  const size_t o_pairs = carve(nrr * sizeof(OvlPair));
+  const size_t o_rl = carve(some(rlist.size()) * 4), o_cl = carve(some(clist.size()) * 4);
+  const size_t o_lda = carve(nref * 4), o_ldb = carve(nref * 4), o_blk = carve((nref + 1) * 4);
+  const size_t o_ps = carve((nref + 1) * 8);
   const size_t o_occa = carve(occ_a.size()), o_occb = carve(occ_b.size());
-  const size_t o_fac = carve(std::max<uint64_t>(1, nfac) * 8), o_u = carve(std::max<uint64_t>(1, nu) * 8);
-  const size_t o_xs = carve(nd * 8), o_part = carve((size_t)pl->nseg * nd * 8);
+  const size_t o_fac = carve(some(nfac) * 8), o_u = carve(some(nu) * 8);
+  const size_t o_xs = carve((pl->nent + 1) * 8);
   const size_t o_t = carve((size_t)nref * nao * nmo * 8), o_o = carve(2 * nrr * n2 * 8);
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && off > free_b) {
@@ -487,37 +725,49 @@ nw_status overlap_plan_get(nw_ctx* ctx, cudaStream_t stream, OverlapPlan** out) 
   pl->ord_det = reinterpret_cast<uint32_t*>(base + o_det);
   pl->ord_a = reinterpret_cast<uint32_t*>(base + o_a_);
   pl->ord_b = reinterpret_cast<uint32_t*>(base + o_b_);
+  pl->ord_e = reinterpret_cast<uint32_t*>(base + o_e_);
   pl->ord_r = reinterpret_cast<double*>(base + o_r_);
-  pl->run_lo = dups ? reinterpret_cast<uint32_t*>(base + o_lo) : nullptr;
-  pl->run_hi = dups ? reinterpret_cast<uint32_t*>(base + o_hi) : nullptr;
+  pl->first = reinterpret_cast<uint32_t*>(base + o_first);
+  pl->tiles = reinterpret_cast<OvlTile*>(base + o_tiles);
   pl->groups = reinterpret_cast<OvlGroup*>(base + o_groups);
   pl->chunks = reinterpret_cast<OvlChunk*>(base + o_chunks);
-  pl->zero_rows = reinterpret_cast<uint64_t*>(base + o_zero);
-  pl->d_a_off = reinterpret_cast<uint64_t*>(base + o_aoff);
-  pl->d_u_off = reinterpret_cast<uint64_t*>(base + o_uoff);
-  pl->d_na = reinterpret_cast<uint32_t*>(base + o_na);
+  pl->src = reinterpret_cast<OvlSource*>(base + o_src);
+  pl->trow = reinterpret_cast<uint32_t*>(base + o_trow);
+  pl->tent = reinterpret_cast<uint32_t*>(base + o_tent);
+  pl->zero_rows = reinterpret_cast<ulonglong2*>(base + o_zero);
+  pl->pairs = reinterpret_cast<OvlPair*>(base + o_pairs);
+  pl->rlist = reinterpret_cast<uint32_t*>(base + o_rl);
+  pl->clist = reinterpret_cast<uint32_t*>(base + o_cl);
+  pl->d_lda = reinterpret_cast<uint32_t*>(base + o_lda);
+  pl->d_ldb = reinterpret_cast<uint32_t*>(base + o_ldb);
+  pl->d_blk = reinterpret_cast<uint32_t*>(base + o_blk);
+  pl->d_pstart = reinterpret_cast<uint64_t*>(base + o_ps);
   uint8_t* d_occa = reinterpret_cast<uint8_t*>(base + o_occa);
   uint8_t* d_occb = reinterpret_cast<uint8_t*>(base + o_occb);
   pl->fac = reinterpret_cast<double*>(base + o_fac);
   pl->u = reinterpret_cast<double*>(base + o_u);
   pl->xs = reinterpret_cast<double*>(base + o_xs);
-  pl->part = reinterpret_cast<double*>(base + o_part);
   double* d_t = reinterpret_cast<double*>(base + o_t);
   double* d_o = reinterpret_cast<double*>(base + o_o);
   auto up = [&](void* dst, const void* src, size_t bytes) {
     return bytes == 0 || cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream) == cudaSuccess;
   };
-  // the padding column of an odd-length B row is summed by stage 1 into a U column nobody reads
-  bool ok = cudaMemsetAsync(pl->fac, 0, std::max<uint64_t>(1, nfac) * 8, stream) == cudaSuccess &&
-            up(pl->ord_det, order.data(), nd * 4) && up(pl->ord_a, o_a.data(), nd * 4) &&
-            up(pl->ord_b, o_b.data(), nd * 4) && up(pl->ord_r, o_r.data(), nd * 8) &&
-            up(pl->groups, groups.data(), groups.size() * sizeof(OvlGroup)) &&
-            up(pl->chunks, chunks.data(), chunks.size() * sizeof(OvlChunk)) &&
-            up(pl->zero_rows, zero_rows.data(), zero_rows.size() * 8) &&
-            up(pl->d_a_off, a_off.data(), nrr * 8) && up(pl->d_u_off, u_off.data(), nrr * 8) &&
-            up(pl->d_na, pl->na.data(), nref * 4) && up(d_occa, occ_a.data(), occ_a.size()) &&
-            up(d_occb, occ_b.data(), occ_b.size());
-  if (ok && dups) ok = up(pl->run_lo, run_lo.data(), nd * 4) && up(pl->run_hi, run_hi.data(), nd * 4);
+  // the padding column of an odd-length table row is summed by stage 1 into a column nobody reads
+  const bool ok_up =
+      up(pl->ord_det, order.data(), nd * 4) && up(pl->ord_a, o_a.data(), nd * 4) && up(pl->ord_b, o_b.data(), nd * 4) &&
+      up(pl->ord_e, o_e.data(), nd * 4) && up(pl->ord_r, o_r.data(), nd * 8) &&
+      up(pl->first, first.data(), first.size() * 4) && up(pl->tiles, tiles.data(), tiles.size() * sizeof(OvlTile)) &&
+      up(pl->groups, groups.data(), groups.size() * sizeof(OvlGroup)) &&
+      up(pl->chunks, chunks.data(), chunks.size() * sizeof(OvlChunk)) &&
+      up(pl->src, src.data(), src.size() * sizeof(OvlSource)) && up(pl->trow, trow.data(), trow.size() * 4) &&
+      up(pl->tent, tent.data(), tent.size() * 4) &&
+      up(pl->zero_rows, zero_rows.data(), zero_rows.size() * sizeof(ulonglong2)) &&
+      up(pl->pairs, pairs.data(), nrr * sizeof(OvlPair)) && up(pl->rlist, rlist.data(), rlist.size() * 4) &&
+      up(pl->clist, clist.data(), clist.size() * 4) && up(pl->d_lda, pl->lda.data(), nref * 4) &&
+      up(pl->d_ldb, pl->ldb.data(), nref * 4) && up(pl->d_blk, blk.data(), blk.size() * 4) &&
+      up(pl->d_pstart, pl->pstart.data(), pl->pstart.size() * 8) && up(d_occa, occ_a.data(), occ_a.size()) &&
+      up(d_occb, occ_b.data(), occ_b.size());
+  bool ok = ok_up && cudaMemsetAsync(pl->fac, 0, some(nfac) * 8, stream) == cudaSuccess;
   // O^{QP}_sigma = C_Q^T (S C_P): nmo x nmo per ordered pair and spin, then the factor tables
   for (int spin = 0; ok && spin < 2 && nref > 1; ++spin) {
     const double* c = spin ? ctx->d_cb : ctx->d_ca;
@@ -541,10 +791,10 @@ nw_status overlap_plan_get(nw_ctx* ctx, cudaStream_t stream, OverlapPlan** out) 
   };
   for (int q = 0; ok && q < nref; ++q)
     for (int p = 0; ok && p < nref; ++p) {
-      if (p == q) continue;
+      if (p == q || pl->pstart[q + 1] == pl->pstart[q]) continue;
       const size_t i = (size_t)q * nref + p;
       factors(d_o + i * n2, d_occa + ca_off[q] * pl->oa, d_occa + ca_off[p] * pl->oa, pl->oa, pl->na[q], pl->na[p],
-              pl->na[q], pl->fac + a_off[i]);
+              pl->lda[q], pl->fac + a_off[i]);
       factors(d_o + (nrr + i) * n2, d_occb + cb_off[q] * pl->ob, d_occb + cb_off[p] * pl->ob, pl->ob, pl->nb[q],
               pl->nb[p], pl->ldb[q], pl->fac + bt_off[i]);
       ok = cudaGetLastError() == cudaSuccess;
@@ -560,27 +810,21 @@ nw_status overlap_plan_get(nw_ctx* ctx, cudaStream_t stream, OverlapPlan** out) 
 }
 
 nw_status overlap_apply(nw_ctx* ctx, const OverlapPlan* pl, const double* x, double* y, cudaStream_t stream) {
-  const uint64_t nd = pl->ndet;
-  ovl_gather_kernel<<<grid_of(nd), kOvlThreads, 0, stream>>>(nd, pl->ord_det, pl->ord_r, x, pl->xs);
-  const int cross = pl->nref > 1 ? 1 : 0;
-  for (int q = 0; cross && q < pl->nref; ++q) {
-    const uint64_t t0 = pl->pstart[q], t1 = pl->pstart[q + 1];
-    if (t1 == t0) continue;
-    const uint32_t ldb = pl->ldb[q];
-    if (pl->nzero[q] > 0)
-      ovl_zero_kernel<<<dim3((unsigned)pl->nzero[q], (ldb + kOvlThreads - 1) / kOvlThreads), kOvlThreads, 0, stream>>>(
-          pl->zero_rows + pl->zero_off[q], ldb, pl->u);
-    if (pl->ngroups[q] > 0)
-      ovl_stage1_kernel<<<dim3((unsigned)pl->ngroups[q], (ldb + 2 * kOvlThreads - 1) / (2 * kOvlThreads)), kOvlThreads, 0,
-                          stream>>>(pl->groups + pl->groups_off[q], pl->chunks, pl->ord_b, pl->xs, pl->fac, ldb, pl->u);
-    const dim3 g2((unsigned)((t1 - t0 + kOvlThreads - 1) / kOvlThreads), (unsigned)pl->nseg);
-    ovl_stage2_kernel<<<g2, kOvlThreads, 0, stream>>>(q, pl->nref, t0, t1, pl->seglen[q], pl->ord_a, pl->ord_b,
-                                                      pl->d_na, pl->d_a_off, pl->d_u_off, pl->na[q], ldb, pl->fac,
-                                                      pl->u, nd,
-                                                      pl->part);
+  ovl_gather_kernel<<<grid_of(pl->nent + 1), kOvlThreads, 0, stream>>>(pl->nent, pl->first, pl->ord_det, pl->ord_r, x,
+                                                                       pl->xs);
+  for (const OverlapPlan::Batch& b : pl->batches) {
+    if (b.nzero > 0)
+      ovl_zero_kernel<<<(unsigned)b.nzero, kOvlThreads, 0, stream>>>(pl->zero_rows + b.zero0, pl->u);
+    if (b.ntile + b.ngroup > 0)
+      ovl_stage1_kernel<<<dim3((unsigned)(b.ntile + b.ngroup), (b.ldmax + 2 * kOvlThreads - 1) / (2 * kOvlThreads)),
+                          kOvlThreads, 0, stream>>>(pl->tiles + b.tile0, (uint32_t)b.ntile, pl->groups + b.group0,
+                                                    pl->chunks, pl->src, pl->trow, pl->tent, pl->xs, pl->fac, pl->u);
+    if (b.nblk > 0)
+      ovl_stage2_kernel<<<b.nblk, kOvlThreads, 0, stream>>>(b.q0, pl->nref, pl->d_blk, pl->d_pstart, pl->pairs,
+                                                            pl->rlist, pl->clist, pl->d_lda, pl->d_ldb, pl->ord_det,
+                                                            pl->ord_a, pl->ord_b, pl->ord_e, pl->ord_r, pl->xs,
+                                                            pl->fac, pl->u, y);
   }
-  ovl_finish_kernel<<<grid_of(nd), kOvlThreads, 0, stream>>>(nd, pl->nseg, cross, pl->ord_det, pl->ord_r, pl->run_lo,
-                                                             pl->run_hi, pl->xs, pl->part, y);
   NW_CUDA(ctx, cudaGetLastError());
   return NW_OK;
 }

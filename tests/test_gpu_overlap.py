@@ -264,3 +264,69 @@ def test_overlap_action_through_quadruple_excitations():
     assert np.abs(y - s @ x).max() <= 1e-13 * scale, np.abs(y - s @ x).max() / scale
     f = OverlapFactorisation(system.s, system.refs, 4, 3, basis)
     assert np.abs(y - f.apply(x)).max() <= 1e-13 * scale
+
+
+def _rows_times_x(w, targets, x):
+    """S[targets] x from the pair evaluator."""
+    nd = x.shape[0]
+    out = np.empty(len(targets))
+    for i, t in enumerate(targets):
+        pairs = np.stack([np.full(nd, t), np.arange(nd)], axis=1).astype(np.uint32)
+        out[i] = w.eval_overlap(pairs) @ x
+    return out
+
+
+@pytest.mark.parametrize("pattern", ["alpha", "beta", "subset", "distinct", "long_row"])
+def test_overlap_action_source_patterns(pattern):
+    """The split of the sources into long rows and long columns on patterns other than a whole singles-and-doubles
+    space: one spin excited only (one column or one row), a random subset, strings that occur once each
+    (every source its own row), and rows longer than a chunk beside tiles with a remainder.  Tolerance as above."""
+    rng = np.random.default_rng(31)
+    system = sy.make_system(13, 3, 3, 3, 20, seed=8, k_scale=0.2)
+    full = sy.sd_basis(13, 3, 3, 3, orders=(1, 2, 4) if pattern == "distinct" else (1, 2))
+    if pattern == "alpha":
+        basis = full[full["rank_b"] == 0]
+    elif pattern == "beta":
+        basis = full[full["rank_a"] == 0]
+    elif pattern == "subset":
+        basis = full[rng.random(full.shape[0]) < 0.3]
+    elif pattern == "distinct":
+        d = full[(full["rank_a"] == 2) & (full["rank_b"] == 2)]
+        n = int(round(np.sqrt((d["parent"] == 0).sum())))    # double strings per spin
+        basis = np.concatenate([d[d["parent"] == p].reshape(n, n)[np.arange(n), rng.permutation(n)] for p in range(3)])
+    else:
+        basis = full[(full["rank_a"] == 0) | ((full["rank_a"] == 1) & (full["rank_b"] == 1)
+                                              & (full["idx_a"][:, 4] < 9))]
+    basis = np.ascontiguousarray(basis)
+    x = rng.standard_normal(basis.shape[0])
+    with nociwick.WicksShared(system.s, system.h, system.eri, system.enuc, system.refs, tol=1e-8) as w:
+        w.build().set_basis(basis)
+        y = _apply(w, x)
+        t = rng.choice(basis.shape[0], 64, replace=False)
+        ref = _rows_times_x(w, t, x)
+    assert np.abs(y[t] - ref).max() <= 1e-13 * np.abs(x).sum(), np.abs(y[t] - ref).max()
+
+
+def test_overlap_action_in_batches_of_targets():
+    """Strings that occur once each make every source its own row: 4 references of 3780 double strings need
+    1.4 GB of single-spin products, more than one batch of target parents holds."""
+    rng = np.random.default_rng(5)
+    system = sy.make_system(40, 4, 4, 4, 20, seed=3, k_scale=0.1)
+    d = sy.sd_basis(40, 4, 4, 1, orders=(2,), include_refs=False)
+    a, b = d[(d["rank_a"] == 2)], d[(d["rank_b"] == 2)]
+    blocks = []
+    for p in range(4):
+        blk = a.copy()
+        k = rng.permutation(b.shape[0])
+        blk["rank_b"], blk["idx_b"] = 2, b["idx_b"][k]
+        blk["phase"] *= b["phase"][k]
+        blk["parent"] = p
+        blocks.append(blk)
+    basis = np.concatenate(blocks)
+    x = rng.standard_normal(basis.shape[0])
+    with nociwick.WicksShared(system.s, system.h, system.eri, system.enuc, system.refs, tol=1e-8) as w:
+        w.build().set_basis(basis)
+        y = _apply(w, x)
+        t = rng.choice(basis.shape[0], 32, replace=False)
+        ref = _rows_times_x(w, t, x)
+    assert np.abs(y[t] - ref).max() <= 1e-13 * np.abs(x).sum(), np.abs(y[t] - ref).max()
