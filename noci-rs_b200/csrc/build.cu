@@ -1166,7 +1166,9 @@ nw_status update_fock(nw_ctx* ctx, const double* fa, const double* fb) {
     cudaFree(ctx->d_fslab);
     ctx->d_fslab = nullptr;
   }
-  if (cudaMalloc(&ctx->d_fslab, sizeof(double) * std::max<size_t>(slab, 32)) != cudaSuccess)
+  const size_t scal_off = (slab + 3) / 4 * 4;  // FsScalars per pair, 32-byte aligned
+  std::vector<FsScalars> scal(npair);
+  if (cudaMalloc(&ctx->d_fslab, sizeof(double) * scal_off + sizeof(FsScalars) * npair) != cudaSuccess)
     return fail(ctx, NW_ERR_ALLOC, "Fock table allocation failed");
   std::vector<FockPair> hfock(npair);
   std::memset(hfock.data(), 0, sizeof(FockPair) * npair);
@@ -1195,6 +1197,9 @@ nw_status update_fock(nw_ctx* ctx, const double* fa, const double* fb) {
       t.f0f[1] = f0f[ps * 2 + 1];
     }
   }
+  for (int p = 0; p < npair; ++p)
+    scal[p] = {hfock[p].a.f0f[0], hfock[p].b.f0f[0], ctx->fast_host[p].a.pref, ctx->fast_host[p].b.pref};
+  NW_CUDA(ctx, cudaMemcpy(ctx->d_fslab + scal_off, scal.data(), sizeof(FsScalars) * npair, cudaMemcpyHostToDevice));
   if (!ctx->d_fockp && cudaMalloc(&ctx->d_fockp, sizeof(FockPair) * npair) != cudaSuccess)
     return fail(ctx, NW_ERR_ALLOC, "Fock table allocation failed");
   NW_CUDA(ctx, cudaMemcpy(ctx->d_fockp, hfock.data(), sizeof(FockPair) * npair, cudaMemcpyHostToDevice));

@@ -492,6 +492,7 @@ EvalParams make_params(const nw_ctx* ctx) {
   P.tol = ctx->tol;
   P.desc = ctx->d_desc;
   P.fock = ctx->d_fockp;
+  P.fslab = ctx->d_fslab;
   P.nbucket = 1;
   P.shift = 0;
   return P;
@@ -703,6 +704,21 @@ nw_status eval_pairs_on(nw_ctx* ctx, EvalParams P, const uint32_t* pairs, uint64
   if (overlap_only) {
     eval_s_kernel<<<grid_stride_blocks(npairs, 128, 16), 128, 0, stream>>>(P, pairs, npairs, out, flag);
     NW_CUDA(ctx, cudaGetLastError());
+    return NW_OK;
+  }
+
+  const bool gen = ctx->nfast < ctx->nresident;
+  if (!(ctx->timing && ctx->serial_classes) && tile_route(P, npairs, mode, gen)) {
+    // phase events: everything is the evaluator's
+    if (ctx->timing)
+      for (int i = 0; i < 4; ++i) NW_CUDA(ctx, cudaEventRecord(ctx->ev[i], stream));
+    NW_CUDA(ctx, eval_tiles(P, reinterpret_cast<const uint2*>(pairs), npairs, out, mode, gen, flag, stream));
+    if (ctx->timing) {
+      for (int i = 4; i < 6; ++i) NW_CUDA(ctx, cudaEventRecord(ctx->ev[i], stream));
+      ctx->timed_gen = false;
+      ctx->timed_classes = false;
+      ctx->timed_valid = true;
+    }
     return NW_OK;
   }
 

@@ -32,6 +32,7 @@ struct EvalParams {
   int32_t exact;
   const uint16_t* desc;    // per-determinant class descriptor (det_desc)
   const FockPair* fock;    // Fock tables (after nw_update_fock), indexed like fast/gen
+  const double* fslab;     // their slab: 8 n^2 doubles per ordered pair, then FsScalars per pair
   uint32_t nbucket;        // sort keys per rank class for fast pairs (pair_sort_key)
   int32_t shift;
   double enuc, tol;
@@ -277,6 +278,13 @@ struct SortScratch {
 // per pair of the request so the counter memset and scan stay small next to the evaluation.
 constexpr uint64_t kFineMax = 1ull << 23;
 constexpr uint64_t kFineMin = 1ull << 14;
+// Largest requests that take the one-kernel evaluation (tile_eval.cu) where the sorted pipeline's order
+// pays for larger ones.  Measured, sorted / one kernel, us: (H, S) at n = 30, 3 references: 512 pairs
+// 37.7 / 10.3, 131072 pairs 51 / 25, 10^6 pairs 109 / 152; n = 64, 6 references: 131072 pairs 76 / 72,
+// 300000 pairs 103 / 153; n = 64 with zero-overlap reference pairs: 131072 pairs 357 / 286, 300000
+// pairs 399 / 574.
+constexpr uint64_t kTileSmallHS = 1ull << 17;
+constexpr uint64_t kTileSmallFS = 1ull << 17;
 
 EvalParams make_params(const nw_ctx* ctx);
 // Number of sort keys with at most `cap` counters for the fast classes; fills P.nbucket/P.shift.
@@ -290,6 +298,12 @@ nw_status launch_sorted(nw_ctx* ctx, const EvalParams& P, uint64_t nkeys, const 
                         double* out, const SortScratch& S, cudaStream_t stream, cudaEvent_t* ev,
                         EvalMode mode = EvalMode::kHS, const uint32_t* npairs_dev = nullptr,
                         bool classified = false);
+
+// One-kernel evaluation of a request (tile_eval.cu): whether `npairs` pairs take it (gen: some resident
+// reference pair has zero-overlap orbitals), and the launch.
+bool tile_route(const EvalParams& P, uint64_t npairs, EvalMode mode, bool gen);
+cudaError_t eval_tiles(const EvalParams& P, const uint2* pairs, uint64_t npairs, double* out, EvalMode mode, bool gen,
+                       uint32_t* flag, cudaStream_t stream);
 
 // Exclusive scan of n counters into offsets[0..n] (offsets[n] = total); tsum holds n / 4096 + 1.
 nw_status scan_exclusive(nw_ctx* ctx, const uint32_t* counts, uint64_t n, uint32_t* offsets, uint32_t* tsum,

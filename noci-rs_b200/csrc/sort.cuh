@@ -11,10 +11,10 @@
 namespace nw {
 
 __device__ __forceinline__ DetRec load_det(const nw_det* dets, uint32_t i) {
-  const ulonglong2* p = reinterpret_cast<const ulonglong2*>(dets + i);
-  const ulonglong2 lo = __ldg(p);
-  const ulonglong2 hi = __ldg(p + 1);
-  return unpack_det(lo.x, lo.y, hi.x, hi.y);
+  // one 32-byte load: a gather costs one tag lookup per lane and instruction
+  uint64_t w0, w1, w2, w3;
+  asm("ld.global.nc.v4.u64 {%0, %1, %2, %3}, [%4];" : "=l"(w0), "=l"(w1), "=l"(w2), "=l"(w3) : "l"(dets + i));
+  return unpack_det(w0, w1, w2, w3);
 }
 
 __device__ __forceinline__ void store_hs(double* out, uint64_t i, double h, double s) {

@@ -94,6 +94,11 @@ struct FockPair {
   FockSpinTab a, b;
 };
 
+// The scalars of one m = 0 (F, S) pair in one 32-byte load: F_0 and the overlap prefactor per spin.
+struct FsScalars {
+  double f0a, f0b, pref_a, pref_b;
+};
+
 
 // ---------------------------------------------------------------------------------------
 // Small determinants.

@@ -1,0 +1,87 @@
+"""One-kernel pair evaluation (small requests; every (F, S) request without zero-overlap reference pairs)
+against the sorted pipeline, which serial class timing selects, and the oracle.
+
+Both routes evaluate the same expressions in FP64; the compiler may contract them differently, so they
+agree to a few roundings of the largest term of an element (1e-12 here: terms of at most about 1e2 for
+these systems, 2^-53 each, a few tens of them), and the oracle to the tolerance of the other parity tests.
+"""
+import numpy as np
+import pytest
+
+import nociwick
+from nociwick import synthetic as sy
+from oracle.oracle import Oracle
+
+pytestmark = pytest.mark.gpu
+ROUTES = 1e-12
+ATOL = 1e-9
+
+
+def _both(w, torch, pairs, fs):
+    stream = torch.cuda.current_stream().cuda_stream
+    dp = torch.from_numpy(np.ascontiguousarray(pairs.astype(np.uint32)).view(np.int32)).cuda()
+    call = w.eval_fs_pairs_device if fs else w.eval_pairs_device
+    outs = []
+    for serial in (False, True):
+        w.set_timing(serial, serial_classes=serial)
+        out = torch.full((pairs.shape[0], 2), float("nan"), dtype=torch.float64, device="cuda")
+        call(dp.data_ptr(), pairs.shape[0], out.data_ptr(), stream)
+        w.sync(stream)
+        outs.append(out.cpu().numpy())
+    w.set_timing(False)
+    return outs
+
+
+@pytest.mark.parametrize("zero_pairs", [[], [(0, 1, 1, 0)], [(0, 1, 0, 2), (1, 2, 1, 1)]])
+@pytest.mark.parametrize("fs", [False, True])
+def test_routes_agree(zero_pairs, fs):
+    """Ranks up to 8 per spin (the runtime path), same-parent pairs beyond doubles, tile and warp edges."""
+    torch = pytest.importorskip("torch")
+    system = sy.make_system(8, 3, 3, 3, 20, seed=1, k_scale=0.3, zero_pairs=zero_pairs, enuc=0.37)
+    basis = sy.sd_basis(8, 3, 3, 3, orders=(1, 2, 3, 4))
+    rng = np.random.default_rng(3)
+    fock = []
+    for _ in range(2):
+        a = rng.normal(0.0, 0.3, (8, 8))
+        fock.append(system.h + 0.5 * (a + a.T))
+    orc = Oracle.from_system(system, tol=1e-8)
+    orc.set_fock(*fock)
+    ob = orc.oracle_basis(basis)
+    with nociwick.WicksShared(system.s, system.h, system.eri, system.enuc, system.refs, tol=1e-8) as w:
+        w.build().set_basis(basis)
+        w.update_fock(*fock)
+        for n in (1, 31, 33, 148 * 32 + 1, 20000, 131072, 131073, 148 * 1024 + 7):
+            pairs = sy.sample_pairs(basis, n, seed=n, distinct_parents=False)
+            one, srt = _both(w, torch, pairs, fs)
+            assert np.all(np.isfinite(one)) and np.max(np.abs(one - srt)) <= ROUTES, n
+            k = min(n, 2000)
+            if fs:
+                _, h_ref, s_ref = orc.eval_m_pairs(ob, pairs[-k:], 0.0)
+            else:
+                h_ref, s_ref = orc.eval_pairs(ob, pairs[-k:])
+            assert np.max(np.abs(one[-k:, 0] - h_ref)) <= ATOL and np.max(np.abs(one[-k:, 1] - s_ref)) <= ATOL, n
+
+
+@pytest.mark.parametrize("fs", [False, True])
+def test_out_of_range_and_one_class(fs):
+    """An index beyond the basis gives NaN and the error, its neighbours their values; a request of one
+    determinant pair repeated fills every tile with one class."""
+    torch = pytest.importorskip("torch")
+    system = sy.make_system(10, 3, 3, 3, 24, seed=7, k_scale=0.3, enuc=0.5)
+    basis = sy.sd_basis(10, 3, 3, 3)
+    per = basis.shape[0] // 3
+    with nociwick.WicksShared(system.s, system.h, system.eri, system.enuc, system.refs, tol=1e-8) as w:
+        w.build().set_basis(basis)
+        w.update_fock(system.h, system.h)
+        pairs = np.tile(np.array([[per - 1, 2 * per - 1]]), (3000, 1))
+        one, srt = _both(w, torch, pairs, fs)
+        assert np.max(np.abs(one - srt)) <= ROUTES and np.all(one == one[0])
+        pairs[1234, 1] = basis.shape[0]
+        stream = torch.cuda.current_stream().cuda_stream
+        dp = torch.from_numpy(pairs.astype(np.uint32).view(np.int32)).cuda()
+        out = torch.zeros((3000, 2), dtype=torch.float64, device="cuda")
+        (w.eval_fs_pairs_device if fs else w.eval_pairs_device)(dp.data_ptr(), 3000, out.data_ptr(), stream)
+        with pytest.raises(nociwick.NwError):
+            w.sync(stream)
+        got = out.cpu().numpy()
+        assert np.all(np.isnan(got[1234])) and np.array_equal(np.delete(got, 1234, 0), np.delete(one, 1234, 0))
