@@ -575,6 +575,8 @@ nw_status nw_ctx_destroy(nw_ctx* ctx) {
   if (ctx->d_fockp) cudaFree(ctx->d_fockp);
   free_buf(ctx->build_work);
   free_buf(ctx->build_tasks);
+  free_buf(ctx->pt2_scratch);
+  free_buf(ctx->pt2_table);
   free_buf(ctx->bt_dets);
   free_buf(ctx->bt_desc);
   free_buf(ctx->bt_pairs);

@@ -92,6 +92,9 @@ struct nw_ctx {
   uint64_t ndet = 0;
   nw::OverlapPlan* ovl = nullptr;  // factor tables of the overlap action, built on first use
 
+  // packed candidate matrix: strings of the candidates, and their pair tables (pt2_strings.cu)
+  nw::DevBuf pt2_scratch, pt2_table;
+
   // evaluation scratch (grown on demand)
   nw::DevBuf keys, perm, counts, offsets, flag, ranks, tsum;
   uint32_t* h_flag = nullptr;      // pinned mirror of the device error flag
@@ -308,6 +311,10 @@ cudaError_t eval_tiles(const EvalParams& P, const uint2* pairs, uint64_t npairs,
 // Exclusive scan of n counters into offsets[0..n] (offsets[n] = total); tsum holds n / 4096 + 1.
 nw_status scan_exclusive(nw_ctx* ctx, const uint32_t* counts, uint64_t n, uint32_t* offsets, uint32_t* tsum,
                          cudaStream_t stream);
+
+// Packed upper triangle of M = F - e0 S over n candidates from single-spin string pairs (pt2_strings.cu),
+// queued on the legacy stream; *done = false where the candidates repeat their strings too little.
+nw_status fill_candidate_m(nw_ctx* ctx, const uint32_t* dcand, uint64_t n, double e0, double* m, bool* done);
 
 // Overlap action y += S x over the resident basis (overlap.cu): the plan (spin components,
 // factor tables, work buffers) is built on first use, allocates and synchronises `stream`, and

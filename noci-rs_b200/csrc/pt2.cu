@@ -4,8 +4,9 @@
 // GMRES, all in FP64.
 //
 //   build     : build_candidate_m / fill_candidate_m (src/snoci/operators.rs:205-296): the upper
-//               triangle of M in packed rows (row a holds M[a][a..n)), from the (F, S) pair
-//               pipeline; the pairs of consecutive rows are exactly consecutive packed entries.
+//               triangle of M in packed rows (row a holds M[a][a..n)), from the candidates'
+//               single-spin string pairs (pt2_strings.cu) where they repeat their strings, else from
+//               the (F, S) pair pipeline; the pairs of consecutive rows are consecutive entries.
 //   mat-vec   : apply_candidate_m (operators.rs:375-488) with the stored matrix: one pass over
 //               the packed triangle in 256 x 256 tiles; a tile adds its row sums to y[rows] and,
 //               off the diagonal, its column sums to y[cols] (FP64 atomics, 512 per tile).  The
@@ -621,6 +622,9 @@ nw_status nw_pt2_create(nw_ctx* ctx, const uint32_t* cand, uint64_t n, double e0
   *out = nullptr;
   if (!ctx || !cand || n == 0 || !std::isfinite(e0)) return NW_ERR_INVALID;
   nw::CtxGuard guard(ctx, nullptr);
+  if (!ctx->built) return nw::fail(ctx, NW_ERR_STATE, "intermediates not built");
+  if (ctx->partial && !ctx->allow_partial)
+    return nw::fail(ctx, NW_ERR_STATE, "the intermediates hold one block of a blocked evaluation (rebuild them)");
   if (!ctx->fock_ready) return nw::fail(ctx, NW_ERR_STATE, "Fock tables not set (nw_update_fock)");
   if (!ctx->d_dets) return nw::fail(ctx, NW_ERR_STATE, "no determinant basis set");
   if (n > 0x7FFFFFFFull) return nw::fail(ctx, NW_ERR_UNSUPPORTED, "too many candidates");
@@ -652,14 +656,19 @@ nw_status nw_pt2_create(nw_ctx* ctx, const uint32_t* cand, uint64_t n, double e0
   if (cudaMalloc(&p->m, sizeof(double) * len) != cudaSuccess || cudaMalloc(&p->mdiag, sizeof(double) * n) != cudaSuccess)
     return cleanup(nw::fail(ctx, NW_ERR_ALLOC, "packed candidate matrix allocation failed (" +
                                                    std::to_string(len * 8 >> 20) + " MiB)"));
-  constexpr uint64_t kBlock = 1ull << 24;  // pairs per evaluation block
-  const uint64_t blk = std::min(kBlock, len);
-  if (cudaMalloc(&dcand, sizeof(uint32_t) * n) != cudaSuccess || cudaMalloc(&pairs, sizeof(uint2) * blk) != cudaSuccess ||
-      cudaMalloc(&fs, sizeof(double2) * blk) != cudaSuccess)
-    return cleanup(nw::fail(ctx, NW_ERR_ALLOC, "candidate pair buffers"));
+  if (cudaMalloc(&dcand, sizeof(uint32_t) * n) != cudaSuccess)
+    return cleanup(nw::fail(ctx, NW_ERR_ALLOC, "candidate buffer"));
   if (cudaMemcpy(dcand, cand, sizeof(uint32_t) * n, cudaMemcpyHostToDevice) != cudaSuccess)
     return cleanup(nw::fail(ctx, NW_ERR_CUDA, "candidate upload"));
-  for (uint64_t base = 0; base < len; base += blk) {
+  bool filled = false;
+  const nw_status fst = nw::fill_candidate_m(ctx, dcand, n, e0, p->m, &filled);
+  if (fst != NW_OK) return cleanup(fst);
+  constexpr uint64_t kBlock = 1ull << 24;  // pairs per evaluation block
+  const uint64_t blk = std::min(kBlock, len);
+  if (!filled && (cudaMalloc(&pairs, sizeof(uint2) * blk) != cudaSuccess ||
+                  cudaMalloc(&fs, sizeof(double2) * blk) != cudaSuccess))
+    return cleanup(nw::fail(ctx, NW_ERR_ALLOC, "candidate pair buffers"));
+  for (uint64_t base = 0; !filled && base < len; base += blk) {
     const uint64_t count = std::min(blk, len - base);
     upper_pairs_kernel<<<grid_n(count), 256>>>(dcand, n, base, count, pairs);
     nw_status st = nw::eval_pairs(ctx, reinterpret_cast<const uint32_t*>(pairs), count, reinterpret_cast<double*>(fs),

@@ -1,0 +1,61 @@
+"""Packed candidate matrix from single-spin string pairs against the dense (F, S) matrices of the pair
+evaluation: products with M over unsorted, repeated and single-parent candidates, ranks up to 4 per spin,
+zero-overlap reference pairs, both conventions, on both sides of the size rule.
+
+An entry is the same expression on both routes, so a product differs by the summation order and a few
+roundings an entry: bound 16 n 2^-53 max_a sum_b |M_ab| |x_b|.
+"""
+import numpy as np
+import pytest
+
+import nociwick
+from nociwick import synthetic as sy
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(w, cand, e0, seed):
+    f, s = w.build_fs_matrix(cand, cand, symmetric=False)
+    up = np.triu(f - e0 * s)
+    m = up + np.triu(up, 1).T
+    rng = np.random.default_rng(seed)
+    with nociwick.Pt2(w, cand, e0) as pt:
+        for _ in range(3):
+            x = rng.normal(size=cand.shape[0])
+            bound = 16 * cand.shape[0] * 2.0 ** -53 * np.max(np.abs(m) @ np.abs(x))
+            assert np.max(np.abs(pt.apply_m(x) - m @ x)) <= bound
+    return m
+
+
+@pytest.mark.parametrize("convention", ["reference", "exact"])
+@pytest.mark.parametrize("zero_pairs", [[], [(0, 1, 1, 0)], [(0, 1, 0, 2), (1, 2, 1, 1)]])
+def test_product_all_ranks(zero_pairs, convention):
+    system = sy.make_system(8, 3, 3, 3, 20, seed=1, k_scale=0.3, zero_pairs=zero_pairs, enuc=0.37)
+    basis = sy.sd_basis(8, 3, 3, 3, orders=(1, 2, 3, 4))
+    rng = np.random.default_rng(5)
+    fa = system.h + np.diag(rng.normal(size=8))
+    fb = system.h - np.diag(rng.normal(size=8))
+    nd = basis.shape[0]
+    with nociwick.WicksShared(system.s, system.h, system.eri, system.enuc, system.refs, tol=1e-8,
+                              convention=convention) as w:
+        w.build().set_basis(basis)
+        w.update_fock(fa, fb)
+        for n in (1023, 1024, 1537):
+            _check(w, rng.choice(nd, n, replace=True).astype(np.uint32), -1.25, n)   # unsorted, repeated
+
+
+def test_single_parent_zeros_and_rule():
+    """One parent: exact zeros beyond doubles; sorted candidates of all parents; too few repeats."""
+    system = sy.make_system(12, 4, 3, 3, 40, seed=2, k_scale=0.3)
+    basis = sy.sd_basis(12, 4, 3, 3)
+    nd = basis.shape[0]
+    per = nd // 3
+    with nociwick.WicksShared(system.s, system.h, system.eri, system.enuc, system.refs, tol=1e-8) as w:
+        w.build().set_basis(basis)
+        w.update_fock(system.h, 0.9 * system.h)
+        m = _check(w, np.arange(per, 2 * per, dtype=np.uint32)[:1100], 0.75, 1)
+        assert (m == 0.0).mean() > 0.1
+        _check(w, np.arange(0, nd, 2, dtype=np.uint32), -0.5, 2)
+        # only doubles in one spin: every candidate has its own string
+        own = np.nonzero((basis["rank_a"] == 2) | (basis["rank_b"] == 2))[0].astype(np.uint32)
+        _check(w, own[:1200], -0.5, 3)
