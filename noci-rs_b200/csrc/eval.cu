@@ -495,6 +495,8 @@ EvalParams make_params(const nw_ctx* ctx) {
   P.fslab = ctx->d_fslab;
   P.nbucket = 1;
   P.shift = 0;
+  P.ngsub = 1;
+  P.gshift = 32;
   return P;
 }
 
@@ -502,14 +504,24 @@ EvalParams make_params(const nw_ctx* ctx) {
 // Fine-key budget: at most kFineMax counters, and at most about one per pair of the request so
 // the counter memset and scan stay small next to the evaluation.
 
-// Number of sort keys for this request with at most `cap` counters for the fast classes;
-// fills P.nbucket / P.shift.
-uint64_t plan_keys(const nw_ctx* ctx, EvalParams& P, uint64_t cap) {
+// Number of sort keys for this request (see internal.cuh).
+uint64_t plan_keys(const nw_ctx* ctx, EvalParams& P, uint64_t cap, uint64_t gen_cap) {
   uint32_t nb = 1;
   P.shift = sort_key_shift(P.ndet, ctx->nref, cap, &nb);
   P.nbucket = nb;
   const uint64_t ngen = (uint64_t)ctx->nresident - (uint64_t)ctx->nfast;
-  return (uint64_t)kClasses * nb + (uint64_t)kGenClasses * ngen;
+  P.ngsub = 1;
+  P.gshift = 32;
+  if (ngen > 0 && P.ndet > 0) {
+    // smallest shift whose sub-buckets fit (2 10^7 pairs at n = 64 with 6 references, a fifth of them m > 0: classify took
+    // 808 us of atomics on 90 busy counters, the whole call 5.06 ms; with sub-buckets 4.58 ms)
+    const uint64_t per = std::max<uint64_t>(1, gen_cap / (kGenClasses * ngen));
+    int g = 0;
+    while (((P.ndet - 1) >> g) + 1 > per) ++g;
+    P.gshift = g;
+    P.ngsub = (uint32_t)(((P.ndet - 1) >> g) + 1);
+  }
+  return (uint64_t)kClasses * nb + (uint64_t)kGenClasses * ngen * P.ngsub;
 }
 
 nw_status scan_exclusive(nw_ctx* ctx, const uint32_t* counts, uint64_t n, uint32_t* offsets, uint32_t* tsum,
@@ -724,7 +736,8 @@ nw_status eval_pairs_on(nw_ctx* ctx, EvalParams P, const uint32_t* pairs, uint64
 
   const uint64_t budget =
       ctx->tune_keys_per_pair > 0.0 ? (uint64_t)(ctx->tune_keys_per_pair * (double)npairs) : std::max(kFineMin, npairs);
-  const uint64_t nkeys = plan_keys(ctx, P, std::min(kFineMax, std::max(kFineMin, budget)));
+  const uint64_t cap = std::min(kFineMax, std::max(kFineMin, budget));
+  const uint64_t nkeys = plan_keys(ctx, P, cap, cap);
   if ((st = ensure(ctx, ctx->keys, npairs * sizeof(uint32_t))) != NW_OK) return st;
   if ((st = ensure(ctx, ctx->ranks, npairs * sizeof(uint32_t))) != NW_OK) return st;
   if ((st = ensure(ctx, ctx->perm, npairs * sizeof(uint32_t))) != NW_OK) return st;
@@ -830,7 +843,7 @@ nw_status eval_pairs_noalloc(nw_ctx* ctx, const uint32_t* pairs, uint64_t npairs
       ctx->tune_keys_per_pair > 0.0 ? (uint64_t)(ctx->tune_keys_per_pair * (double)npairs) : std::max(kFineMin, npairs);
   const uint64_t fast_cap = std::min(kNoallocMaxKeys - (uint64_t)kGenClasses * ngen,
                                      std::min(kFineMax, std::max(kFineMin, budget)));
-  const uint64_t nkeys = plan_keys(ctx, P, fast_cap);
+  const uint64_t nkeys = plan_keys(ctx, P, fast_cap, 0);
   if (nkeys > kNoallocMaxKeys) return fail(ctx, NW_ERR_UNSUPPORTED, "sort keys exceed the allocation-free scratch");
   SortScratch S;
   S.keys = reinterpret_cast<uint32_t*>(base + kNoallocOffKeys);

@@ -35,6 +35,8 @@ struct EvalParams {
   const double* fslab;     // their slab: 8 n^2 doubles per ordered pair, then FsScalars per pair
   uint32_t nbucket;        // sort keys per rank class for fast pairs (pair_sort_key)
   int32_t shift;
+  uint32_t ngsub;          // bra sub-buckets of a zero-overlap class
+  int32_t gshift;
   double enuc, tol;
 };
 
@@ -290,8 +292,9 @@ constexpr uint64_t kTileSmallHS = 1ull << 17;
 constexpr uint64_t kTileSmallFS = 1ull << 17;
 
 EvalParams make_params(const nw_ctx* ctx);
-// Number of sort keys with at most `cap` counters for the fast classes; fills P.nbucket/P.shift.
-uint64_t plan_keys(const nw_ctx* ctx, EvalParams& P, uint64_t cap);
+// Number of sort keys with at most `cap` counters for the fast classes and at most gen_cap for the
+// zero-overlap ones (at least one a class); fills P.nbucket / P.shift and P.ngsub / P.gshift.
+uint64_t plan_keys(const nw_ctx* ctx, EvalParams& P, uint64_t cap, uint64_t gen_cap);
 // classify -> scan -> scatter -> evaluate on `stream` (no allocation, no host synchronisation).
 // With npairs_dev the number of pairs is read on the device (at most npairs, the capacity the
 // launch is sized for); ev (eight events or null) brackets the phases.  With classified the

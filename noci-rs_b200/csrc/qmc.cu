@@ -898,7 +898,8 @@ nw_status nw_qmc_create(nw_ctx* ctx, const nw_qmc_opts* opts, const double* c0, 
   // scans all keys, and finer buckets gain the evaluators less than the scan costs), not from
   // the attempt capacity
   const uint64_t typical = (uint64_t)(0.25 * std::max(opts->target_population, opts->initial_population)) + nd;
-  q->nkeys = nw::plan_keys(ctx, q->P, std::min<uint64_t>(nw::kFineMax, std::max<uint64_t>(nw::kFineMin, std::min(typical, cap))));
+  const uint64_t key_cap = std::min<uint64_t>(nw::kFineMax, std::max<uint64_t>(nw::kFineMin, std::min(typical, cap)));
+  q->nkeys = nw::plan_keys(ctx, q->P, key_cap, key_cap);
   take(q->S.keys, cap);
   take(q->S.ranks, cap);
   take(q->S.sidx, cap);

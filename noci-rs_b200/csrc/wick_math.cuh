@@ -921,18 +921,21 @@ NW_HD int rank_class(int la, int lb) { return (la <= 4 && lb <= 4) ? la * 5 + lb
 // working set nref times smaller in L2.  Pairs of reference pairs with zero-overlap orbitals follow,
 // keyed by (sort position - nfast, L_alpha, L_beta) with the full ranks 0..kML: their
 // distribution sums cost about L^7 per spin, so a warp whose lanes mixed ranks would run every
-// lane at the pace of its largest L.  Keys are < kRankClasses * nbucket + kGenClasses *
-// (nref^2 - nfast).
+// lane at the pace of its largest L.  Each of those classes has ngsub sub-buckets by bra, for the
+// lanes of a warp to share the bra's rows and for the counters' sake (a few hundred counters for
+// millions of pairs serialise their atomics).  Keys are < kRankClasses * nbucket + kGenClasses *
+// (nref^2 - nfast) * ngsub.
 // ---------------------------------------------------------------------------------------
 constexpr int kRankClasses = 26;
 constexpr int kGenClasses = (kML + 1) * (kML + 1);
 
 NW_HD uint32_t pair_sort_key(int la, int lb, uint32_t bra, int ket_parent, int ord, int nfast, uint64_t ndet,
-                             uint32_t nbucket, int shift) {
+                             uint32_t nbucket, int shift, uint32_t ngsub = 1, int gshift = 32) {
   if (ord < nfast)
     return (uint32_t)rank_class(la, lb) * nbucket +
            (uint32_t)((((uint64_t)ket_parent * ndet) + bra) >> shift);
-  return (uint32_t)kRankClasses * nbucket + (uint32_t)((ord - nfast) * kGenClasses + la * (kML + 1) + lb);
+  return (uint32_t)kRankClasses * nbucket +
+         (uint32_t)((ord - nfast) * kGenClasses + la * (kML + 1) + lb) * ngsub + (uint32_t)((uint64_t)bra >> gshift);
 }
 
 // Smallest shift for which the fast-pair keys, kRankClasses * nbucket, fit in cap (cap >= 26).
