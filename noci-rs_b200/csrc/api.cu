@@ -112,7 +112,7 @@ nw_status eval_hs_pipelined(nw_ctx* ctx, nw::EvalMode mode, const uint32_t* pair
   for (cudaStream_t q : {ctx->s_in, ctx->s_comp, ctx->s_out}) NW_CUDA(ctx, cudaStreamWaitEvent(q, ctx->ev_start, 0));
   NW_CUDA(ctx, cudaMemsetAsync(flag, 0, sizeof(uint32_t), ctx->s_comp));
   uint64_t chunk = (npairs + nw::kPipeChunks - 1) / nw::kPipeChunks;
-  chunk = std::max<uint64_t>(nw::kPipeMinChunk, (chunk + 255) / 256 * 256);
+  chunk = std::max<uint64_t>(nw::pipe_min_chunk(ctx), (chunk + 255) / 256 * 256);
   uint64_t k = 0;
   for (uint64_t o = 0; o < npairs; o += chunk, ++k) {
     const uint64_t nk = std::min(chunk, npairs - o);
@@ -160,7 +160,7 @@ nw_status eval_host(nw_ctx* ctx, nw::EvalMode mode, const uint32_t* pairs_host, 
   if ((st = nw::ensure(ctx, ctx->io_hs, npairs * 2 * sizeof(double))) != NW_OK) return st;
   uint32_t* dp = static_cast<uint32_t*>(ctx->io_pairs.p);
   double* dh = static_cast<double*>(ctx->io_hs.p);
-  if (npairs >= 2 * nw::kPipeMinChunk && is_pinned(pairs_host) && is_pinned(out_host))
+  if (npairs >= 2 * nw::pipe_min_chunk(ctx) && is_pinned(pairs_host) && is_pinned(out_host))
     return eval_hs_pipelined(ctx, mode, pairs_host, npairs, out_host, dp, dh, s);
   NW_CUDA(ctx, cudaMemcpyAsync(dp, pairs_host, npairs * 2 * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
   if ((st = nw::eval_pairs(ctx, dp, npairs, dh, mode, s)) != NW_OK) return st;

@@ -85,3 +85,19 @@ def test_out_of_range_and_one_class(fs):
             w.sync(stream)
         got = out.cpu().numpy()
         assert np.all(np.isnan(got[1234])) and np.array_equal(np.delete(got, 1234, 0), np.delete(one, 1234, 0))
+
+
+@pytest.mark.parametrize("zero_pairs", [[], [(0, 1, 1, 0)]])
+def test_pinned_host_chunks(zero_pairs):
+    """Pinned host buffers around the smallest pipelined request, chunks of whole and ragged size."""
+    torch = pytest.importorskip("torch")
+    system = sy.make_system(10, 3, 3, 3, 24, seed=7, k_scale=0.3, enuc=0.5, zero_pairs=zero_pairs)
+    basis = sy.sd_basis(10, 3, 3, 3)
+    with nociwick.WicksShared(system.s, system.h, system.eri, system.enuc, system.refs, tol=1e-8) as w:
+        w.build().set_basis(basis)
+        for n in ((1 << 17) - 1, 1 << 17, 200_001, 600_001):
+            pairs = sy.sample_pairs(basis, n, seed=n, distinct_parents=False)
+            host = torch.from_numpy(pairs.astype(np.uint32).view(np.int32)).pin_memory()
+            out = torch.full((n, 2), float("nan"), dtype=torch.float64).pin_memory()
+            w.eval_pairs(host.numpy().view(np.uint32), out.numpy())
+            assert np.max(np.abs(out.numpy() - _both(w, torch, pairs, False)[0])) <= ROUTES, n
