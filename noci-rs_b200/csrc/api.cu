@@ -23,13 +23,24 @@ nw_status cuda_fail(nw_ctx* ctx, cudaError_t e, const char* what) {
   return fail(ctx, NW_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
+cudaError_t ctx_malloc(nw_ctx* ctx, void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && ctx->pt2_spare.p) {
+    cudaGetLastError();
+    cudaFree(ctx->pt2_spare.p);
+    ctx->pt2_spare = DevBuf{};
+    e = cudaMalloc(p, bytes);
+  }
+  return e;
+}
+
 nw_status ensure(nw_ctx* ctx, DevBuf& b, size_t bytes) {
   if (b.bytes >= bytes) return NW_OK;
   if (b.p) cudaFree(b.p);
   b.p = nullptr;
   b.bytes = 0;
   size_t want = bytes + bytes / 4 + 256;
-  cudaError_t e = cudaMalloc(&b.p, want);
+  cudaError_t e = ctx_malloc(ctx, &b.p, want);
   if (e != cudaSuccess) {
     b.p = nullptr;
     return fail(ctx, NW_ERR_ALLOC, std::string("scratch allocation failed: ") + cudaGetErrorString(e));
@@ -239,7 +250,7 @@ nw_status create_base(int nao, int nmo, double enuc, const double* s, const doub
   if (st == NW_OK) st = upload(ctx, &ctx->d_h, h, n2);
   if (st == NW_OK) st = upload(ctx, &ctx->d_ca, refs->c_alpha, (size_t)nref * nao * nmo);
   if (st == NW_OK) st = upload(ctx, &ctx->d_cb, refs->c_beta, (size_t)nref * nao * nmo);
-  if (st == NW_OK && cudaMallocHost(&ctx->h_flag, sizeof(uint32_t)) != cudaSuccess) st = NW_ERR_ALLOC;
+  if (st == NW_OK && cudaMallocHost(&ctx->h_flag, 64) != cudaSuccess) st = NW_ERR_ALLOC;
   for (int i = 0; i < 3 && st == NW_OK; ++i)
     if (cudaStreamCreateWithFlags(&ctx->s_aux[i], cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_join[i], cudaEventDisableTiming) != cudaSuccess)
@@ -577,6 +588,8 @@ nw_status nw_ctx_destroy(nw_ctx* ctx) {
   free_buf(ctx->build_tasks);
   free_buf(ctx->pt2_scratch);
   free_buf(ctx->pt2_table);
+  free_buf(ctx->pt2_spare);
+  free_buf(ctx->gmres_work);
   free_buf(ctx->bt_dets);
   free_buf(ctx->bt_desc);
   free_buf(ctx->bt_pairs);

@@ -878,7 +878,7 @@ nw_status build_all(nw_ctx* ctx, const std::vector<char>* subset) {
   }
   {
     if (!ctx->d_slab) {
-      cudaError_t e = cudaMalloc(&ctx->d_slab, slab_need);
+      cudaError_t e = ctx_malloc(ctx, reinterpret_cast<void**>(&ctx->d_slab), slab_need);
       if (e != cudaSuccess) {
         ctx->d_slab = nullptr;
         return fail(ctx, NW_ERR_ALLOC, "intermediate slab allocation failed (" +

@@ -96,10 +96,12 @@ struct nw_ctx {
 
   // packed candidate matrix: strings of the candidates, and their pair tables (pt2_strings.cu)
   nw::DevBuf pt2_scratch, pt2_table;
+  nw::DevBuf pt2_spare;            // matrix of the last destroyed operator (at most kKeepMatrix bytes)
+  nw::DevBuf gmres_work;           // vectors and scratch of the solves (kept up to kKeepGmres bytes)
 
   // evaluation scratch (grown on demand)
   nw::DevBuf keys, perm, counts, offsets, flag, ranks, tsum;
-  uint32_t* h_flag = nullptr;      // pinned mirror of the device error flag
+  uint32_t* h_flag = nullptr;      // pinned: mirror of the device error flag; words 4, 5: GMRES steps
   nw::DevBuf io_pairs, io_hs;      // staging for the host-buffer entry point
   // determinant records, descriptors and pairs packed from caller excitation caches
   // (nw_eval_hs_batched), and their device staging for host-buffer calls
@@ -183,6 +185,13 @@ inline uint64_t pipe_min_chunk(const nw_ctx* ctx) { return ctx->nfast < ctx->nre
 nw_status fail(nw_ctx* ctx, nw_status st, const std::string& msg);
 nw_status cuda_fail(nw_ctx* ctx, cudaError_t e, const char* what);
 nw_status ensure(nw_ctx* ctx, DevBuf& b, size_t bytes);
+// cudaMalloc that gives back the context's spare candidate matrix before it fails.
+cudaError_t ctx_malloc(nw_ctx* ctx, void** p, size_t bytes);
+
+// What a context keeps between candidate operators: allocating and freeing their matrix and vectors took
+// longer than the solve itself (12000 candidates, 576 MB: 2.2 of 4.4 ms).
+constexpr size_t kKeepMatrix = 1ull << 30;
+constexpr size_t kKeepGmres = 256ull << 20;
 
 // Row-major, strided-batched FP64 GEMM on the FP64 tensor cores (dgemm.cu):
 // C[b] (M x N) = alpha op(A[b]) op(B[b]) + beta C[b], op(X) = X^T when the flag is set

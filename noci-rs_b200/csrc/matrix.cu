@@ -74,7 +74,7 @@ struct DevMem {
 };
 
 nw_status dev_alloc(nw_ctx* ctx, DevMem& m, size_t bytes, const char* what) {
-  if (cudaMalloc(&m.p, std::max<size_t>(bytes, 256)) != cudaSuccess) {
+  if (ctx_malloc(ctx, &m.p, std::max<size_t>(bytes, 256)) != cudaSuccess) {
     m.p = nullptr;
     return fail(ctx, NW_ERR_ALLOC, std::string(what) + ": device allocation failed");
   }

@@ -716,7 +716,7 @@ nw_status overlap_plan_get(nw_ctx* ctx, cudaStream_t stream, OverlapPlan** out) 
     return fail(ctx, NW_ERR_ALLOC,
                 "the overlap factor tables need " + std::to_string(off >> 20) + " MiB, more than the free device memory");
   }
-  if (cudaMalloc(&pl->mem, off) != cudaSuccess) {
+  if (ctx_malloc(ctx, reinterpret_cast<void**>(&pl->mem), off) != cudaSuccess) {
     pl->mem = nullptr;
     overlap_plan_free(pl);
     return fail(ctx, NW_ERR_ALLOC, "overlap factor table allocation failed");

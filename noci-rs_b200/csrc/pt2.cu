@@ -23,8 +23,7 @@
 //               rotations, back substitution, restart from the true residual; convergence on
 //               |r| / sqrt(n) <= res_tol.  Each Arnoldi step runs on the device (own two-pass
 //               reduction kernels; the Hessenberg matrix, rotations and stopping rule in device
-//               memory); on the packed path the step is one CUDA graph, replayed for every step
-//               of a cycle without host synchronisation (one per restart cycle).
+//               memory); the host queues one step ahead of the one whose stopping flag it reads.
 //   precond   : Preconditioner::new / apply (src/snoci/types.rs:161-288): diagonal inverse with
 //               the reference's floor, and the Woodbury rank-2 correction for the projection.
 #include <cuda_runtime.h>
@@ -33,6 +32,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstddef>
+#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -272,12 +272,12 @@ __global__ void mul_kernel(const double* __restrict__ a, const double* __restric
 inline int grid_n(uint64_t n) { return (int)std::min<uint64_t>((n + 255) / 256, 148 * 16); }
 
 // ---------------------------------------------------------------------------------------
-// Device-side Arnoldi step of GMRES (one CUDA graph per solve on the packed path).  The
+// Device-side Arnoldi step of GMRES.  The
 // scalars of the cycle live on the device (ArnoldiState, the Hessenberg matrix, the Givens
 // rotations and the rotated right-hand side g); every reduction is two-pass and in a fixed
 // order (per-block partial sums, then one ordered sum), and every kernel returns at once when
-// the cycle is done, so the host can queue the `inner` steps of a cycle back to back and
-// synchronise once per cycle (gmres.rs:197-266 for the rotations and the stopping rule).
+// the cycle is done, so the host can queue a step before it knows whether the previous one
+// was the last (gmres.rs:197-266 for the rotations and the stopping rule).
 // ---------------------------------------------------------------------------------------
 constexpr int kVB = 256;            // threads of the vector kernels
 constexpr int kVBlocks = 148 * 4;   // blocks of the vector kernels = partial sums per reduction
@@ -528,7 +528,8 @@ struct nw_pt2 {
   uint64_t n = 0;
   double e0 = 0.0;
   double* m = nullptr;      // packed upper triangle, n (n + 1) / 2 (null when matrix-free)
-  double* mdiag = nullptr;  // diagonal of M
+  size_t m_bytes = 0;       // allocated at m
+  double* mdiag = nullptr;  // diagonal of M, then the vectors of nw_pt2_apply_m (3 n)
   float last_symv_ms = 0.0f;
   // matrix-free mode: candidates, and one block of upper-triangle pairs and their (F, S)
   uint32_t* dcand = nullptr;
@@ -653,10 +654,19 @@ nw_status nw_pt2_create(nw_ctx* ctx, const uint32_t* cand, uint64_t n, double e0
     }
     return st;
   };
-  if (cudaMalloc(&p->m, sizeof(double) * len) != cudaSuccess || cudaMalloc(&p->mdiag, sizeof(double) * n) != cudaSuccess)
+  // the spare matrix of the context, unless much of it would lie idle
+  p->m_bytes = sizeof(double) * len;
+  if (ctx->pt2_spare.bytes >= p->m_bytes && ctx->pt2_spare.bytes / 4 <= p->m_bytes) {
+    p->m = static_cast<double*>(ctx->pt2_spare.p);
+    p->m_bytes = ctx->pt2_spare.bytes;
+    ctx->pt2_spare = nw::DevBuf{};
+  } else if (nw::ctx_malloc(ctx, reinterpret_cast<void**>(&p->m), p->m_bytes) != cudaSuccess) {
+    p->m = nullptr;
+  }
+  if (!p->m || nw::ctx_malloc(ctx, reinterpret_cast<void**>(&p->mdiag), sizeof(double) * 3 * n) != cudaSuccess)
     return cleanup(nw::fail(ctx, NW_ERR_ALLOC, "packed candidate matrix allocation failed (" +
                                                    std::to_string(len * 8 >> 20) + " MiB)"));
-  if (cudaMalloc(&dcand, sizeof(uint32_t) * n) != cudaSuccess)
+  if (nw::ctx_malloc(ctx, reinterpret_cast<void**>(&dcand), sizeof(uint32_t) * n) != cudaSuccess)
     return cleanup(nw::fail(ctx, NW_ERR_ALLOC, "candidate buffer"));
   if (cudaMemcpy(dcand, cand, sizeof(uint32_t) * n, cudaMemcpyHostToDevice) != cudaSuccess)
     return cleanup(nw::fail(ctx, NW_ERR_CUDA, "candidate upload"));
@@ -665,8 +675,8 @@ nw_status nw_pt2_create(nw_ctx* ctx, const uint32_t* cand, uint64_t n, double e0
   if (fst != NW_OK) return cleanup(fst);
   constexpr uint64_t kBlock = 1ull << 24;  // pairs per evaluation block
   const uint64_t blk = std::min(kBlock, len);
-  if (!filled && (cudaMalloc(&pairs, sizeof(uint2) * blk) != cudaSuccess ||
-                  cudaMalloc(&fs, sizeof(double2) * blk) != cudaSuccess))
+  if (!filled && (nw::ctx_malloc(ctx, reinterpret_cast<void**>(&pairs), sizeof(uint2) * blk) != cudaSuccess ||
+                  nw::ctx_malloc(ctx, reinterpret_cast<void**>(&fs), sizeof(double2) * blk) != cudaSuccess))
     return cleanup(nw::fail(ctx, NW_ERR_ALLOC, "candidate pair buffers"));
   for (uint64_t base = 0; !filled && base < len; base += blk) {
     const uint64_t count = std::min(blk, len - base);
@@ -709,9 +719,10 @@ nw_status nw_pt2_create_matrix_free(nw_ctx* ctx, const uint32_t* cand, uint64_t 
     if (st != NW_OK) nw_pt2_destroy(p);
     return st;
   };
-  if (cudaMalloc(&p->dcand, sizeof(uint32_t) * n) != cudaSuccess || cudaMalloc(&p->mdiag, sizeof(double) * n) != cudaSuccess ||
-      cudaMalloc(&p->pairs, sizeof(uint2) * p->blk) != cudaSuccess ||
-      cudaMalloc(&p->fs, sizeof(double2) * p->blk) != cudaSuccess)
+  if (nw::ctx_malloc(ctx, reinterpret_cast<void**>(&p->dcand), sizeof(uint32_t) * n) != cudaSuccess ||
+      nw::ctx_malloc(ctx, reinterpret_cast<void**>(&p->mdiag), sizeof(double) * 3 * n) != cudaSuccess ||
+      nw::ctx_malloc(ctx, reinterpret_cast<void**>(&p->pairs), sizeof(uint2) * p->blk) != cudaSuccess ||
+      nw::ctx_malloc(ctx, reinterpret_cast<void**>(&p->fs), sizeof(double2) * p->blk) != cudaSuccess)
     return cleanup(nw::fail(ctx, NW_ERR_ALLOC, "matrix-free candidate buffers"));
   if (cudaMemcpy(p->dcand, cand, sizeof(uint32_t) * n, cudaMemcpyHostToDevice) != cudaSuccess)
     return cleanup(nw::fail(ctx, NW_ERR_CUDA, "candidate upload"));
@@ -731,11 +742,7 @@ nw_status nw_pt2_apply_m(nw_pt2* p, const double* x, double* y) {
   nw::CtxGuard guard(p->ctx, nullptr);
   nw_ctx* ctx = p->ctx;
   NW_CUDA(ctx, cudaSetDevice(ctx->device));
-  double *dx = nullptr, *dy = nullptr;
-  if (cudaMalloc(&dx, sizeof(double) * p->n) != cudaSuccess || cudaMalloc(&dy, sizeof(double) * p->n) != cudaSuccess) {
-    if (dx) cudaFree(dx);
-    return pfail(p, NW_ERR_ALLOC, "vector allocation");
-  }
+  double *dx = p->mdiag + p->n, *dy = dx + p->n;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
@@ -750,8 +757,6 @@ nw_status nw_pt2_apply_m(nw_pt2* p, const double* x, double* y) {
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  cudaFree(dx);
-  cudaFree(dy);
   if (st != NW_OK) return st;
   if (e != cudaSuccess) return nw::cuda_fail(ctx, e, "candidate mat-vec");
   return NW_OK;
@@ -775,12 +780,21 @@ nw_status nw_pt2_solve(nw_pt2* p, const nw_pt2_projection* proj, const double* r
   const int kmax = opts->restart;
   // device vectors: 4 projection, dinv, z0, z1, b, x, r, w, z, Krylov basis (kmax + 1)
   const uint64_t nvec = 12 + (uint64_t)kmax + 1;
-  double* base = nullptr;
-  if (cudaMalloc(&base, sizeof(double) * n * nvec) != cudaSuccess) return pfail(p, NW_ERR_ALLOC, "GMRES vectors");
-  struct Free {
-    double* q;
-    ~Free() { cudaFree(q); }
-  } free_base{base};
+  const int ld = kmax + 1;
+  const size_t nscr = (size_t)kVBlocks * ld + 4 * (size_t)kVBlocks + 2 * (size_t)ld + (size_t)(kmax + 1) * kmax +
+                      2 * (size_t)kmax + (size_t)ld;
+  static_assert(sizeof(ArnoldiState) % sizeof(double) == 0, "state before the scratch");
+  if (nw::ensure(ctx, ctx->gmres_work, sizeof(double) * (n * nvec + nscr) + sizeof(ArnoldiState)) != NW_OK)
+    return pfail(p, NW_ERR_ALLOC, "GMRES vectors");
+  struct Shrink {
+    nw::DevBuf& b;
+    ~Shrink() {
+      if (b.bytes <= nw::kKeepGmres) return;
+      cudaFree(b.p);
+      b = nw::DevBuf{};
+    }
+  } shrink{ctx->gmres_work};
+  double* base = static_cast<double*>(ctx->gmres_work.p);
   auto vec = [&](int i) { return base + (uint64_t)i * n; };
   double *s_a0 = vec(0), *s_0a = vec(1), *f_a0 = vec(2), *f_0a = vec(3), *dinv = vec(4), *z0 = vec(5), *z1 = vec(6);
   double *b = vec(7), *x = vec(8), *r = vec(9), *w = vec(10), *z = vec(11), *Q = vec(12);
@@ -848,25 +862,22 @@ nw_status nw_pt2_solve(nw_pt2* p, const nw_pt2_projection* proj, const double* r
 
   // device-side Arnoldi scratch: the cycle state, per-block partial sums, Gram-Schmidt
   // coefficients, the Hessenberg matrix, rotations and g
-  const int ld = kmax + 1;
-  const size_t nscr = (size_t)kVBlocks * ld + 4 * (size_t)kVBlocks + 2 * (size_t)ld + (size_t)(kmax + 1) * kmax +
-                      2 * (size_t)kmax + (size_t)ld;
   struct ArnoldiRes {
-    void* mem = nullptr;
     cudaStream_t q = nullptr;
-    cudaGraphExec_t exec = nullptr;
+    cudaEvent_t step[2] = {nullptr, nullptr};
+    int* done = nullptr;  // pinned, one word per step in flight
     ~ArnoldiRes() {
-      if (exec) cudaGraphExecDestroy(exec);
+      for (cudaEvent_t e : step)
+        if (e) cudaEventDestroy(e);
       if (q) cudaStreamDestroy(q);
-      if (mem) cudaFree(mem);
     }
   } ar;
-  if (cudaMalloc(&ar.mem, sizeof(ArnoldiState) + sizeof(double) * nscr) != cudaSuccess)
-    return pfail(p, NW_ERR_ALLOC, "GMRES Arnoldi scratch");
   // a blocking stream: ordered with the legacy-stream work (products, cuBLAS) around it
   NW_CUDA(ctx, cudaStreamCreate(&ar.q));
-  ArnoldiState* dst = static_cast<ArnoldiState*>(ar.mem);
-  double* part = reinterpret_cast<double*>(static_cast<char*>(ar.mem) + sizeof(ArnoldiState));
+  for (cudaEvent_t& e : ar.step) NW_CUDA(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  ar.done = reinterpret_cast<int*>(ctx->h_flag) + 4;
+  ArnoldiState* dst = reinterpret_cast<ArnoldiState*>(base + n * nvec);
+  double* part = reinterpret_cast<double*>(dst + 1);
   double* part_a = part + (size_t)kVBlocks * ld;      // 2 per block
   double* part_b = part_a + 2 * (size_t)kVBlocks;     // 2 per block
   double* coef = part_b + 2 * (size_t)kVBlocks;
@@ -904,21 +915,6 @@ nw_status nw_pt2_solve(nw_pt2* p, const nw_pt2_projection* proj, const double* r
     NW_CUDA(ctx, cudaGetLastError());
     return NW_OK;
   };
-  if (p->m) {
-    // the packed path's step is one CUDA graph, captured once per solve and replayed per step
-    cudaGraph_t graph = nullptr;
-    NW_CUDA(ctx, cudaStreamBeginCapture(ar.q, cudaStreamCaptureModeThreadLocal));
-    const nw_status cst = enqueue_step(ar.q);
-    const cudaError_t ce = cudaStreamEndCapture(ar.q, &graph);
-    if (cst != NW_OK) {
-      if (graph) cudaGraphDestroy(graph);
-      return cst;
-    }
-    NW_CUDA(ctx, ce);
-    const cudaError_t ie = cudaGraphInstantiate(&ar.exec, graph, 0);
-    cudaGraphDestroy(graph);
-    NW_CUDA(ctx, ie);
-  }
   while (!converged && total < opts->max_iter) {
     PT_BLAS(p, cublasDnrm2(h, (int)n, r, 1, &beta));
     if (beta <= kSmall) {
@@ -932,18 +928,20 @@ nw_status nw_pt2_solve(nw_pt2* p, const nw_pt2_projection* proj, const double* r
     PT_BLAS(p, cublasDscal(h, (int)n, &inv, Q, 1));
     arn_init_kernel<<<1, kVB, 0, ar.q>>>(dst, inner, opts->res_tol * rms, beta, kmax, dH, dg);
     NW_CUDA(ctx, cudaGetLastError());
-    if (ar.exec) {
-      // every step of the cycle queued at once; the steps after the stopping point are no-ops
-      for (int k = 0; k < inner; ++k) NW_CUDA(ctx, cudaGraphLaunch(ar.exec, ar.q));
-    } else {
-      for (int k = 0; k < inner; ++k) {
+    // One step is queued beyond the one whose outcome the host waits for, so the device never idles and at
+    // most one step after the stopping point runs, as no-ops.  (Queueing all `inner` steps of a cycle that
+    // stops early as graphs cost 0.4 ms of empty launches and the capture, of a 2.9 ms solve.)
+    const int ahead = p->m ? 1 : 0;
+    for (int k = 0; k < inner + ahead; ++k) {
+      if (k < inner) {
         nw_status st = enqueue_step(ar.q);
         if (st != NW_OK) return st;
-        int done = 0;
-        NW_CUDA(ctx, cudaMemcpyAsync(&done, done_flag, sizeof(int), cudaMemcpyDeviceToHost, ar.q));
-        NW_CUDA(ctx, cudaStreamSynchronize(ar.q));
-        if (done) break;
+        NW_CUDA(ctx, cudaMemcpyAsync(ar.done + (k & 1), done_flag, sizeof(int), cudaMemcpyDeviceToHost, ar.q));
+        NW_CUDA(ctx, cudaEventRecord(ar.step[k & 1], ar.q));
       }
+      if (k < ahead) continue;
+      NW_CUDA(ctx, cudaEventSynchronize(ar.step[(k - ahead) & 1]));
+      if (ar.done[(k - ahead) & 1]) break;
     }
     NW_CUDA(ctx, cudaStreamSynchronize(ar.q));
     ArnoldiState hst;
@@ -984,6 +982,17 @@ nw_status nw_pt2_destroy(nw_pt2* p) {
   if (!p) return NW_OK;
   cudaSetDevice(p->ctx->device);
   cudaDeviceSynchronize();
+  if (p->m && p->m_bytes <= nw::kKeepMatrix) {
+    // the larger of this matrix and the spare one stays with the context
+    std::lock_guard<std::recursive_mutex> lock(p->ctx->mtx);
+    nw::DevBuf& spare = p->ctx->pt2_spare;
+    if (p->m_bytes > spare.bytes) {
+      if (spare.p) cudaFree(spare.p);
+      spare.p = p->m;
+      spare.bytes = p->m_bytes;
+      p->m = nullptr;
+    }
+  }
   for (void* q : {(void*)p->m, (void*)p->mdiag, (void*)p->dcand, (void*)p->pairs, (void*)p->fs})
     if (q) cudaFree(q);
   delete p;

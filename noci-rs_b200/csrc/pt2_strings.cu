@@ -367,7 +367,7 @@ nw_status fill_candidate_m(nw_ctx* ctx, const uint32_t* dcand, uint64_t n, doubl
   if (ctx->pt2_table.bytes < tab_bytes) {
     if (ctx->pt2_table.p) cudaFree(ctx->pt2_table.p);
     ctx->pt2_table = DevBuf{};
-    if (cudaMalloc(&ctx->pt2_table.p, tab_bytes) != cudaSuccess) {
+    if (ctx_malloc(ctx, &ctx->pt2_table.p, tab_bytes) != cudaSuccess) {
       cudaGetLastError();
       ctx->pt2_table.p = nullptr;
       return NW_OK;   // no room: the pair pipeline builds M

@@ -117,9 +117,9 @@ __device__ __forceinline__ double learned_pgen(const QmcParams& q, const Proposa
 }
 
 template <class T>
-T* dalloc(size_t count, bool* ok) {
+T* dalloc(nw_ctx* ctx, size_t count, bool* ok) {
   void* p = nullptr;
-  if (cudaMalloc(&p, std::max<size_t>(count * sizeof(T), 256)) != cudaSuccess) {
+  if (nw::ctx_malloc(ctx, &p, std::max<size_t>(count * sizeof(T), 256)) != cudaSuccess) {
     *ok = false;
     return nullptr;
   }
@@ -871,7 +871,7 @@ nw_status nw_qmc_create(nw_ctx* ctx, const nw_qmc_opts* opts, const double* c0, 
   bool ok = true;
   auto take = [&](auto*& p, size_t count) {
     using T = std::remove_reference_t<decltype(*p)>;
-    p = dalloc<T>(count, &ok);
+    p = dalloc<T>(ctx, count, &ok);
     q->owned.push_back(p);
   };
   take(q->st, 1);

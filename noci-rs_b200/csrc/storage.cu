@@ -318,7 +318,7 @@ nw_status load_intermediates(nw_ctx* ctx, const char* slab_path, const char* met
   ctx->slab_capacity = 0;
   if (ctx->d_fbase) cudaFree(ctx->d_fbase);
   ctx->d_fbase = nullptr;
-  if (cudaMalloc(&ctx->d_slab, std::max<size_t>(hd.slab_bytes, 256)) != cudaSuccess) {
+  if (ctx_malloc(ctx, reinterpret_cast<void**>(&ctx->d_slab), std::max<size_t>(hd.slab_bytes, 256)) != cudaSuccess) {
     ctx->d_slab = nullptr;
     return fail(ctx, NW_ERR_ALLOC, "intermediate slab allocation failed");
   }

@@ -59,3 +59,45 @@ def test_single_parent_zeros_and_rule():
         # only doubles in one spin: every candidate has its own string
         own = np.nonzero((basis["rank_a"] == 2) | (basis["rank_b"] == 2))[0].astype(np.uint32)
         _check(w, own[:1200], -0.5, 3)
+
+
+def test_matrix_and_vectors_kept_between_operators():
+    """Operators of other sizes made, used and destroyed in turn on one context, two alive at once: the kept
+    matrix and GMRES vectors hold nothing of an earlier operator."""
+    system = sy.make_system(12, 4, 3, 3, 40, seed=2, k_scale=0.3)
+    basis = sy.sd_basis(12, 4, 3, 3)
+    nd = basis.shape[0]
+    rng = np.random.default_rng(1)
+
+    def product(w, cand, x):
+        with nociwick.Pt2(w, cand, -0.5) as pt:
+            return pt.apply_m(x)
+
+    sizes = (1500, 700, 1600, 1500)
+    cands = [rng.choice(nd, n, replace=False).astype(np.uint32) for n in sizes]
+    xs = [rng.normal(size=n) for n in sizes]
+    fresh, solved = [], []
+    opts = dict(max_iter=12, restart=5, res_tol=1e-10)
+
+    def solve(pt, n, x):
+        z = np.zeros(n)
+        return pt.solve(0.0, z, z, z, z, x, **opts)
+
+    for cand, x in zip(cands, xs):
+        with nociwick.WicksShared(system.s, system.h, system.eri, system.enuc, system.refs, tol=1e-8) as w:
+            w.build().set_basis(basis)
+            w.update_fock(system.h, system.h)
+            fresh.append(product(w, cand, x))
+            with nociwick.Pt2(w, cand, -0.5) as pt:
+                solved.append(solve(pt, cand.shape[0], x))
+    with nociwick.WicksShared(system.s, system.h, system.eri, system.enuc, system.refs, tol=1e-8) as w:
+        w.build().set_basis(basis)
+        w.update_fock(system.h, system.h)
+        for cand, x, y, (sx, si) in zip(cands, xs, fresh, solved):
+            # column sums reach y by FP64 atomics in no fixed order
+            assert np.max(np.abs(product(w, cand, x) - y)) <= 1e-11 * max(1.0, np.max(np.abs(y)))
+            with nociwick.Pt2(w, cand, -0.5) as pt, nociwick.Pt2(w, cands[1], -0.5) as other:
+                gx, gi = solve(pt, cand.shape[0], x)
+                assert gi["iterations"] == si["iterations"]
+                assert np.max(np.abs(gx - sx)) <= 1e-6 * max(1.0, np.max(np.abs(sx)))
+                assert np.max(np.abs(other.apply_m(xs[1]) - fresh[1])) <= 1e-11 * max(1.0, np.max(np.abs(fresh[1])))
