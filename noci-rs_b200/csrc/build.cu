@@ -44,13 +44,14 @@ inline cudaError_t gemm_b(cudaStream_t h, bool ta, bool tb, int M, int N, int K,
   return dgemm_strided(h, ta, tb, M, N, K, alpha, A, lda, sa, B, ldb, sb, beta, C, ldc, sc, batch);
 }
 
-// y[b][i] += alpha x[b][i] for a batch of vectors at strides sx, sy.
-__global__ void axpy_batched_kernel(double alpha, const double* __restrict__ x, long long sx, double* __restrict__ y,
-                                    long long sy, long long n) {
-  const double* xb = x + blockIdx.y * sx;
-  double* yb = y + blockIdx.y * sy;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    yb[i] += alpha * xb[i];
+// Y^(0) = X^(0) - T, Y^(1) = X^(1) per (pair, spin), with T = rowc^T S colc held in the second half of Y.
+__global__ void y_kernel(const double* __restrict__ X, long long n2, double* __restrict__ Y) {
+  const double* x = X + blockIdx.y * 2 * n2;
+  double* y = Y + blockIdx.y * 2 * n2;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n2; i += (long long)gridDim.x * blockDim.x) {
+    y[i] = x[i] + -1.0 * y[n2 + i];
+    y[n2 + i] = x[n2 + i];
+  }
 }
 
 // Bump allocator over one device buffer, 256-byte aligned pieces.
@@ -270,15 +271,29 @@ __global__ void transpose_kernel(const double* __restrict__ src, int n, double* 
   }
 }
 
-// Fast-layout records: recx = {X0, hcol0}, recy = {Y0, hcol0}.
-__global__ void records_kernel(const double* __restrict__ X0, const double* __restrict__ Y0,
-                               const double* __restrict__ F, const double* __restrict__ V,
-                               const double* __restrict__ Vd, int n, double2* __restrict__ recx,
-                               double2* __restrict__ recy) {
+// The n x n pieces of the slab in one launch, blockIdx.y = piece: fast-layout records recx = {X0, hcol0},
+// recy = {Y0, hcol0} (src0..4 = X0, Y0, F, V, V_diff), a transposed copy, or a copy.
+enum PieceKind { kPieceRecords = 0, kPieceTranspose = 1, kPieceCopy = 2 };
+struct PieceTask {
+  const double* src[5];
+  double* dst[2];
+  int kind;
+  int pad;
+};
+
+__global__ void pieces_kernel(const PieceTask* __restrict__ tasks, int n) {
+  const PieceTask& t = tasks[blockIdx.y];
   for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n * n; idx += gridDim.x * blockDim.x) {
-    const double hc = F[idx] + V[idx] + Vd[idx];
-    recx[idx] = make_double2(X0[idx], hc);
-    recy[idx] = make_double2(Y0[idx], hc);
+    if (t.kind == kPieceRecords) {
+      const double hc = t.src[2][idx] + t.src[3][idx] + t.src[4][idx];
+      reinterpret_cast<double2*>(t.dst[0])[idx] = make_double2(t.src[0][idx], hc);
+      reinterpret_cast<double2*>(t.dst[1])[idx] = make_double2(t.src[1][idx], hc);
+    } else if (t.kind == kPieceTranspose) {
+      // the scattered side is the read, which the caches hold
+      t.dst[0][idx] = t.src[0][(size_t)(idx % n) * n + idx / n];
+    } else {
+      t.dst[0][idx] = t.src[0][idx];
+    }
   }
 }
 
@@ -697,73 +712,74 @@ nw_status build_all(nw_ctx* ctx, const std::vector<char>* subset) {
 
   // ---------------- dense products ----------------
   const int B2 = nps * 2;  // (ps, m)
-  // MtS = M^T S, MS = M S
-  NW_DG(ctx, gemm_b(h, true, false, n, n, n, 1.0, M, n, n2, ctx->d_s, n, 0, 0.0, MtS, n, n2, B2));
-  NW_DG(ctx, gemm_b(h, false, false, n, n, n, 1.0, M, n, n2, ctx->d_s, n, 0, 0.0, MS, n, n2, B2));
-  // products with the per-ps C copies, one call per m
+  // Products of one dependency level run as one launch (dgemm_group): n = 30 and 3 references took 45
+  // launches of 18 to 36 single-tile products, 5.6 us each.
+  const long long q2 = (long long)n2;
+  std::vector<GemmGroup> lv;
+  auto add = [&](const double* A, long long sa, const double* B, long long sb, double* C, long long sc, int batch) {
+    lv.push_back(GemmGroup{A, B, C, sa, sb, sc, batch});
+  };
+  auto run = [&](bool ta) {
+    const cudaError_t e = dgemm_group(h, ta, n, lv.data(), (int)lv.size());
+    lv.clear();
+    return e;
+  };
+  // MtS = M^T S, tmp(ps, 0) = rowc^T S (for Y); MS = M S
+  add(M, q2, ctx->d_s, 0, MtS, q2, B2);
+  add(rowc, q2, ctx->d_s, 0, Y, 2 * q2, nps);  // held in Y until X is known
+  NW_DG(ctx, run(true));
+  add(M, q2, ctx->d_s, 0, MS, q2, B2);
+  NW_DG(ctx, run(false));
+  // products with the per-ps C copies; S M S; rowc^T S colc
   for (int m = 0; m < 2; ++m) {
     const size_t off = (size_t)m * n2;
-    NW_DG(ctx, gemm_b(h, false, false, n, n, n, 1.0, MtS + off, n, 2 * n2, cxs, n, n2, 0.0, mtsx + off, n, 2 * n2, nps));
-    NW_DG(ctx, gemm_b(h, false, false, n, n, n, 1.0, MtS + off, n, 2 * n2, cws, n, n2, 0.0, mtsw + off, n, 2 * n2, nps));
-    NW_DG(ctx, gemm_b(h, false, false, n, n, n, 1.0, MS + off, n, 2 * n2, cxs, n, n2, 0.0, msx + off, n, 2 * n2, nps));
-    NW_DG(ctx, gemm_b(h, false, false, n, n, n, 1.0, MS + off, n, 2 * n2, cws, n, n2, 0.0, msw + off, n, 2 * n2, nps));
+    add(MtS + off, 2 * q2, cxs, q2, mtsx + off, 2 * q2, nps);
+    add(MtS + off, 2 * q2, cws, q2, mtsw + off, 2 * q2, nps);
+    add(MS + off, 2 * q2, cxs, q2, msx + off, 2 * q2, nps);
+    add(MS + off, 2 * q2, cws, q2, msw + off, 2 * q2, nps);
   }
+  add(ctx->d_s, 0, MS, q2, tmp, q2, B2);
+  add(Y, 2 * q2, colc, q2, Y + n2, 2 * q2, nps);
+  NW_DG(ctx, run(false));
   cxxc_kernel<<<dim3(grid_for(n2) > 64 ? 64 : grid_for(n2), B2), 256>>>(mtsx, mtsw, msx, msw, cxs, cws, nao, n, oa, ob,
                                                                       cx, xc);
   NW_CUDA(ctx, cudaGetLastError());
-  // X^(m) = rowc^T (S M S) colc: tmp = MS * S; X = rowc^T tmp colc
-  NW_DG(ctx, gemm_b(h, false, false, n, n, n, 1.0, ctx->d_s, n, 0, MS, n, n2, 0.0, tmp, n, n2, B2));  // S M S
-  for (int m = 0; m < 2; ++m) {
-    const size_t off = (size_t)m * n2;
-    NW_DG(ctx, gemm_b(h, true, false, n, n, n, 1.0, rowc, n, n2, tmp + off, n, 2 * n2, 0.0, MS + off, n, 2 * n2, nps));
-    NW_DG(ctx, gemm_b(h, false, false, n, n, n, 1.0, MS + off, n, 2 * n2, colc, n, n2, 0.0, X + off, n, 2 * n2, nps));
-  }
-  // Y^(0) = X^(0) - rowc^T S colc, Y^(1) = X^(1): tmp(ps,0) = rowc^T S, tmp(ps,1) = tmp(ps,0) colc
-  NW_DG(ctx, gemm_b(h, true, false, n, n, n, 1.0, rowc, n, n2, ctx->d_s, n, 0, 0.0, tmp, n, 2 * n2, nps));
-  NW_DG(ctx, gemm_b(h, false, false, n, n, n, 1.0, tmp, n, 2 * n2, colc, n, n2, 0.0, tmp + n2, n, 2 * n2, nps));
-  NW_CUDA(ctx, cudaMemcpyAsync(Y, X, sizeof(double) * nps * 2 * n2, cudaMemcpyDeviceToDevice));
-  // Y(ps,0) -= tmp(ps,1)
-  axpy_batched_kernel<<<dim3(grid_for(n2) > 64 ? 64 : grid_for(n2), nps), 256>>>(-1.0, tmp + n2, 2 * (long long)n2, Y,
-                                                                              2 * (long long)n2, (long long)n2);
+  // X^(m) = rowc^T (S M S) colc
+  for (int m = 0; m < 2; ++m) add(rowc, q2, tmp + m * n2, 2 * q2, MS + m * n2, 2 * q2, nps);
+  NW_DG(ctx, run(true));
+  // ... and hxc[ps][mj] = h xc[mj]
+  for (int m = 0; m < 2; ++m) add(MS + m * n2, 2 * q2, colc, q2, X + m * n2, 2 * q2, nps);
+  add(ctx->d_h, 0, xc, q2, hxc, q2, B2);
+  NW_DG(ctx, run(false));
+  // Y^(0) = X^(0) - rowc^T S colc, Y^(1) = X^(1)
+  y_kernel<<<dim3(grid_for(n2) > 64 ? 64 : grid_for(n2), nps), 256>>>(X, q2, Y);
   NW_CUDA(ctx, cudaGetLastError());
-  // JK and Coulomb-only J for all (ps, m): rows of M are vec(M)
+  // JK and Coulomb-only J for all (ps, m): rows of M are vec(M); the four-index scratch is free here
   g_kernel<<<grid_for(n4), 256>>>(ctx->d_eri, n, G);
   NW_CUDA(ctx, cudaGetLastError());
-  NW_DG(ctx, gemm(h, false, true, B2, (int)n2, (int)n2, 1.0, M, (int)n2, G, (int)n2, 0.0, JK, (int)n2));
-  NW_DG(ctx, gemm(h, false, true, B2, (int)n2, (int)n2, 1.0, M, (int)n2, ctx->d_eri, (int)n2, 0.0, Jc, (int)n2));
-  // hxc[ps][mj] = h xc[mj]; Fh[ps][mi][mj] = cx[mi]^T hxc[mj]
-  NW_DG(ctx, gemm_b(h, false, false, n, n, n, 1.0, ctx->d_h, n, 0, xc, n, n2, 0.0, hxc, n, n2, B2));
-  for (int mi = 0; mi < 2; ++mi)
-    for (int mj = 0; mj < 2; ++mj)
-      NW_DG(ctx, gemm_b(h, true, false, n, n, n, 1.0, cx + mi * n2, n, 2 * n2, hxc + mj * n2, n, 2 * n2, 0.0,
-                          Fh + (size_t)(mi * 2 + mj) * n2, n, 4 * n2, nps));
-  // JKxc[ps][mk][mj] = JK[mk] xc[mj]; V[ps][mi][mj][mk] = cx[mi]^T JKxc[mk][mj]
+  NW_DG(ctx, dgemm_nt_pair(h, B2, (int)n2, (int)n2, M, G, JK, ctx->d_eri, Jc, tA, tensors));
+  // JKxc[ps][mk][mj] = JK[mk] xc[mj].  Different-spin: JcXc[ps][mo][mk] = Jc_other[mo] xc_this[mk], for
+  // alpha (ps = 2p) the other spin's Jc follows, for beta it precedes.
   for (int mk = 0; mk < 2; ++mk)
-    for (int mj = 0; mj < 2; ++mj)
-      NW_DG(ctx, gemm_b(h, false, false, n, n, n, 1.0, JK + mk * n2, n, 2 * n2, xc + mj * n2, n, 2 * n2, 0.0,
-                          JKxc + (size_t)(mk * 2 + mj) * n2, n, 4 * n2, nps));
-  for (int mi = 0; mi < 2; ++mi)
-    for (int mj = 0; mj < 2; ++mj)
-      for (int mk = 0; mk < 2; ++mk)
-        NW_DG(ctx, gemm_b(h, true, false, n, n, n, 1.0, cx + mi * n2, n, 2 * n2, JKxc + (size_t)(mk * 2 + mj) * n2, n,
-                            4 * n2, 0.0, Vv + (size_t)((mi * 2 + mj) * 2 + mk) * n2, n, 8 * n2, nps));
-  // Different-spin: for alpha (ps = 2p) vab[ma0][mb0][mak] = cx_a[ma0]^T Jc_b[mb0] xc_a[mak];
-  // for beta (ps = 2p+1) vba[mb0][ma0][mbk] = cx_b[mb0]^T Jc_a[ma0] xc_b[mbk].
-  // JcXc[ps][mo][mk] = Jc_other[mo] xc_this[mk]
-  for (int mo = 0; mo < 2; ++mo)
-    for (int mk = 0; mk < 2; ++mk) {
-      // alpha rows: other = beta (ps+1)
-      NW_DG(ctx, gemm_b(h, false, false, n, n, n, 1.0, Jc + 2 * n2 + mo * n2, n, 4 * n2, xc + mk * n2, n, 4 * n2, 0.0,
-                          JcXc + (size_t)(mo * 2 + mk) * n2, n, 8 * n2, npair));
-      // beta rows: other = alpha (ps-1)
-      NW_DG(ctx, gemm_b(h, false, false, n, n, n, 1.0, Jc + mo * n2, n, 4 * n2, xc + 2 * n2 + mk * n2, n, 4 * n2, 0.0,
-                          JcXc + 4 * n2 + (size_t)(mo * 2 + mk) * n2, n, 8 * n2, npair));
+    for (int mj = 0; mj < 2; ++mj) {
+      add(JK + mk * n2, 2 * q2, xc + mj * n2, 2 * q2, JKxc + (size_t)(mk * 2 + mj) * n2, 4 * q2, nps);
+      add(Jc + 2 * n2 + mk * n2, 4 * q2, xc + mj * n2, 4 * q2, JcXc + (size_t)(mk * 2 + mj) * n2, 8 * q2, npair);
+      add(Jc + mk * n2, 4 * q2, xc + 2 * n2 + mj * n2, 4 * q2, JcXc + 4 * n2 + (size_t)(mk * 2 + mj) * n2, 8 * q2, npair);
     }
-  for (int mt = 0; mt < 2; ++mt)
-    for (int mo = 0; mo < 2; ++mo)
-      for (int mk = 0; mk < 2; ++mk)
-        NW_DG(ctx, gemm_b(h, true, false, n, n, n, 1.0, cx + mt * n2, n, 2 * n2, JcXc + (size_t)(mo * 2 + mk) * n2, n,
-                            4 * n2, 0.0, Vd + (size_t)((mt * 2 + mo) * 2 + mk) * n2, n, 8 * n2, nps));
+  NW_DG(ctx, run(false));
+  // Fh[ps][mi][mj] = cx[mi]^T hxc[mj]; V[ps][mi][mj][mk] = cx[mi]^T JKxc[mk][mj];
+  // alpha vab[ma0][mb0][mak] = cx_a[ma0]^T Jc_b[mb0] xc_a[mak], beta vba[mb0][ma0][mbk] likewise.
+  for (int mi = 0; mi < 2; ++mi)
+    for (int mj = 0; mj < 2; ++mj) {
+      add(cx + mi * n2, 2 * q2, hxc + mj * n2, 2 * q2, Fh + (size_t)(mi * 2 + mj) * n2, 4 * q2, nps);
+      for (int mk = 0; mk < 2; ++mk) {
+        add(cx + mi * n2, 2 * q2, JKxc + (size_t)(mk * 2 + mj) * n2, 4 * q2, Vv + (size_t)((mi * 2 + mj) * 2 + mk) * n2,
+            8 * q2, nps);
+        add(cx + mi * n2, 2 * q2, JcXc + (size_t)(mj * 2 + mk) * n2, 4 * q2, Vd + (size_t)((mi * 2 + mj) * 2 + mk) * n2,
+            8 * q2, nps);
+      }
+    }
+  NW_DG(ctx, run(true));
 
   // ---------------- scalars ----------------
   // per ps: f0h[2] = tr(M[m] h), v0 terms tr(JK0 M0), tr(JK0 M1), tr(JK1 M1);
@@ -898,6 +914,10 @@ nw_status build_all(nw_ctx* ctx, const std::vector<char>* subset) {
   std::memset(hgen.data(), 0, sizeof(GenPair) * npair);
   auto CX = [&](int ps, int m) { return cx + ((size_t)ps * 2 + m) * n2; };
   auto XC = [&](int ps, int m) { return xc + ((size_t)ps * 2 + m) * n2; };
+  std::vector<PieceTask> pieces;
+  auto piece = [&](PieceKind kind, const double* src, double* dst) {
+    pieces.push_back(PieceTask{{src, nullptr, nullptr, nullptr, nullptr}, {dst, nullptr}, kind, 0});
+  };
   FusedPlan plan;
   for (int p = 0; p < npair; ++p) {
     if (!resident(p)) continue;
@@ -913,9 +933,11 @@ nw_status build_all(nw_ctx* ctx, const std::vector<char>* subset) {
         const int ps = 2 * p + s;
         double2* recx = reinterpret_cast<double2*>(S0 + fo[p].recx[s]);
         double2* recy = reinterpret_cast<double2*>(S0 + fo[p].recy[s]);
-        records_kernel<<<g2, 256>>>(X + (size_t)ps * 2 * n2, Y + (size_t)ps * 2 * n2, Fh + (size_t)ps * 4 * n2,
-                                    Vv + (size_t)ps * 8 * n2, Vd + (size_t)ps * 8 * n2, n, recx, recy);
-        NW_CUDA(ctx, cudaGetLastError());
+        pieces.push_back(PieceTask{{X + (size_t)ps * 2 * n2, Y + (size_t)ps * 2 * n2, Fh + (size_t)ps * 4 * n2,
+                                    Vv + (size_t)ps * 8 * n2, Vd + (size_t)ps * 8 * n2},
+                                   {S0 + fo[p].recx[s], S0 + fo[p].recy[s]},
+                                   kPieceRecords,
+                                   0});
         if (!fused) {
           nw_status st = transform4(ctx, ctx->d_eri, n, CX(ps, 0), XC(ps, 0), CX(ps, 0), XC(ps, 0), tA, tD, cwp);
           if (st != NW_OK) return st;
@@ -948,20 +970,19 @@ nw_status build_all(nw_ctx* ctx, const std::vector<char>* subset) {
         const int ms = hmeta[ps].m;
         GenSpin& gs = s ? gp.b : gp.a;
         for (int m = 0; m < 2; ++m) {
-          NW_CUDA(ctx, cudaMemcpyAsync(S0 + g.x[s][m], X + ((size_t)ps * 2 + m) * n2, n2 * 8, cudaMemcpyDeviceToDevice));
-          NW_CUDA(ctx, cudaMemcpyAsync(S0 + g.y[s][m], Y + ((size_t)ps * 2 + m) * n2, n2 * 8, cudaMemcpyDeviceToDevice));
+          piece(kPieceCopy, X + ((size_t)ps * 2 + m) * n2, S0 + g.x[s][m]);
+          piece(kPieceCopy, Y + ((size_t)ps * 2 + m) * n2, S0 + g.y[s][m]);
           gs.x[m] = S0 + g.x[s][m];
           gs.y[m] = S0 + g.y[s][m];
         }
         for (int k = 0; k < 4; ++k) {
-          transpose_kernel<<<g2, 256>>>(Fh + ((size_t)ps * 4 + k) * n2, n, S0 + g.fh[s][k]);
+          piece(kPieceTranspose, Fh + ((size_t)ps * 4 + k) * n2, S0 + g.fh[s][k]);
           gs.fh_t[k >> 1][k & 1] = S0 + g.fh[s][k];
         }
         for (int k = 0; k < 8; ++k) {
-          transpose_kernel<<<g2, 256>>>(Vv + ((size_t)ps * 8 + k) * n2, n, S0 + g.v[s][k]);
+          piece(kPieceTranspose, Vv + ((size_t)ps * 8 + k) * n2, S0 + g.v[s][k]);
           gs.v_t[k >> 2][(k >> 1) & 1][k & 1] = S0 + g.v[s][k];
         }
-        NW_CUDA(ctx, cudaGetLastError());
         static const int br[10][4] = {{0, 0, 0, 0}, {0, 0, 0, 1}, {0, 0, 1, 0}, {0, 0, 1, 1}, {0, 1, 0, 1},
                                       {0, 1, 1, 0}, {0, 1, 1, 1}, {1, 0, 1, 0}, {1, 0, 1, 1}, {1, 1, 1, 1}};
         for (int sl = 0; sl < 10; ++sl) {
@@ -994,12 +1015,11 @@ nw_status build_all(nw_ctx* ctx, const std::vector<char>* subset) {
         gs.m = ms;
       }
       for (int k = 0; k < 8; ++k) {
-        transpose_kernel<<<g2, 256>>>(Vd + ((size_t)psa * 8 + k) * n2, n, S0 + g.vab[k]);
-        transpose_kernel<<<g2, 256>>>(Vd + ((size_t)psb * 8 + k) * n2, n, S0 + g.vba[k]);
+        piece(kPieceTranspose, Vd + ((size_t)psa * 8 + k) * n2, S0 + g.vab[k]);
+        piece(kPieceTranspose, Vd + ((size_t)psb * 8 + k) * n2, S0 + g.vba[k]);
         gp.vab_t[k >> 2][(k >> 1) & 1][k & 1] = S0 + g.vab[k];
         gp.vba_t[k >> 2][(k >> 1) & 1][k & 1] = S0 + g.vba[k];
       }
-      NW_CUDA(ctx, cudaGetLastError());
       for (int k = 0; k < 16; ++k) {
         const int a0 = (k >> 3) & 1, az = (k >> 2) & 1, b0 = (k >> 1) & 1, by = k & 1;
         if (g.ii[k] == (size_t)-1) {
@@ -1022,6 +1042,15 @@ nw_status build_all(nw_ctx* ctx, const std::vector<char>* subset) {
           gp.vba0[j][i] = tr_p[4 + j * 2 + i];
         }
     }
+  }
+
+  for (size_t i = 0; i < pieces.size(); i += 65535) {  // grid.y
+    const std::vector<PieceTask> part(pieces.begin() + i, pieces.begin() + std::min(pieces.size(), i + 65535));
+    PieceTask* d = nullptr;
+    const nw_status st = upload_tasks(ctx, part, &d);
+    if (st != NW_OK) return st;
+    pieces_kernel<<<dim3(std::min(g2, 16), (unsigned)part.size()), 256>>>(d, n);
+    NW_CUDA(ctx, cudaGetLastError());
   }
 
   if (fused) {

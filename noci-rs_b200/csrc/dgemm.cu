@@ -18,6 +18,8 @@
 // (a shared operand).
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "internal.cuh"
 
 namespace nw {
@@ -95,18 +97,15 @@ __device__ __forceinline__ void load_panels(const GemmArgs& g, const double* A, 
   }
 }
 
+// The C tile at (m0, n0) of one product over the K panels kt0 .. kt1 - 1.
 template <bool TA, bool TB>
-__global__ void __launch_bounds__(kThreads) dgemm_kernel(GemmArgs g) {
+__device__ __forceinline__ void gemm_tile(const GemmArgs& g, const double* __restrict__ A, const double* __restrict__ B,
+                                          double* __restrict__ C, int m0, int n0, int kt0, int kt1) {
   extern __shared__ __align__(16) double dsm[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
   const int grp = lane >> 2, tig = lane & 3;
-  const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * kBN;
-  const long long bz = blockIdx.z;
-  const double* __restrict__ A = g.A + bz * g.sa;
-  const double* __restrict__ B = g.B + bz * g.sb;
-  double* __restrict__ C = g.C + bz * g.sc;
-  const int nk = (g.K + kBK - 1) / kBK;
+  const int nk = kt1 - kt0;
 
   double acc[2][4][4];
 #pragma unroll
@@ -118,7 +117,7 @@ __global__ void __launch_bounds__(kThreads) dgemm_kernel(GemmArgs g) {
 
 #pragma unroll
   for (int s = 0; s < kStages - 1; ++s) {
-    if (s < nk) load_panels<TA, TB>(g, A, B, m0, n0, s, dsm + (2 * s) * kPanel, dsm + (2 * s + 1) * kPanel);
+    if (s < nk) load_panels<TA, TB>(g, A, B, m0, n0, kt0 + s, dsm + (2 * s) * kPanel, dsm + (2 * s + 1) * kPanel);
     cp_async_commit();
   }
   for (int kt = 0; kt < nk; ++kt) {
@@ -126,7 +125,7 @@ __global__ void __launch_bounds__(kThreads) dgemm_kernel(GemmArgs g) {
     __syncthreads();               // ... and every thread's; stage (kt - 1) % kStages is free
     {
       const int nx = kt + kStages - 1, st = nx % kStages;
-      if (nx < nk) load_panels<TA, TB>(g, A, B, m0, n0, nx, dsm + (2 * st) * kPanel, dsm + (2 * st + 1) * kPanel);
+      if (nx < nk) load_panels<TA, TB>(g, A, B, m0, n0, kt0 + nx, dsm + (2 * st) * kPanel, dsm + (2 * st + 1) * kPanel);
       cp_async_commit();
     }
     const int st = kt % kStages;
@@ -166,18 +165,78 @@ __global__ void __launch_bounds__(kThreads) dgemm_kernel(GemmArgs g) {
 }
 
 template <bool TA, bool TB>
-cudaError_t launch(cudaStream_t stream, const GemmArgs& g, dim3 grid) {
-  // the three-stage ring is above the 48 KB default; raised once per device
-  static bool raised[64] = {};
+__global__ void __launch_bounds__(kThreads) dgemm_kernel(GemmArgs g) {
+  const long long bz = blockIdx.z;
+  gemm_tile<TA, TB>(g, g.A + bz * g.sa, g.B + bz * g.sb, g.C + bz * g.sc, blockIdx.y * kBM, blockIdx.x * kBN, 0,
+                    (g.K + kBK - 1) / kBK);
+}
+
+// Batches of one shape in one launch: blockIdx.z = entry * most + batch index.
+struct GroupArgs {
+  GemmGroup e[kGemmGroupMax];
+  int most, n;
+};
+
+template <bool TA>
+__global__ void __launch_bounds__(kThreads) dgemm_group_kernel(const __grid_constant__ GroupArgs g) {
+  const int q = blockIdx.z / g.most, z = blockIdx.z - q * g.most;
+  const GemmGroup& e = g.e[q];
+  if (z >= e.batch) return;
+  const GemmArgs a{nullptr, nullptr, nullptr, 0, 0, 0, g.n, g.n, g.n, g.n, g.n, g.n, 1.0, 0.0};
+  gemm_tile<TA, false>(a, e.A + z * e.sa, e.B + z * e.sb, e.C + z * e.sc, blockIdx.y * kBM, blockIdx.x * kBN, 0,
+                       (g.n + kBK - 1) / kBK);
+}
+
+// C_h[split] = A B_h^T over the split's K panels, h = 0, 1: blockIdx.z = h * splits + split.
+__global__ void __launch_bounds__(kThreads) dgemm_split_kernel(GemmArgs g, const double* __restrict__ B1, int splits,
+                                                               int per) {
+  const int h = blockIdx.z / splits, sp = blockIdx.z - h * splits;
+  const int nk = (g.K + kBK - 1) / kBK;
+  gemm_tile<false, true>(g, g.A, h ? B1 : g.B, g.C + blockIdx.z * g.sc, blockIdx.y * kBM, blockIdx.x * kBN, sp * per,
+                         min(nk, (sp + 1) * per));
+}
+
+// The splits' partial products in order.
+__global__ void split_sum_kernel(const double* __restrict__ part, int splits, long long len, double* __restrict__ C0,
+                                 double* __restrict__ C1) {
+  double* C = blockIdx.y ? C1 : C0;
+  const double* p = part + blockIdx.y * splits * len;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < len; i += (long long)gridDim.x * blockDim.x) {
+    double v = p[i];
+    for (int s = 1; s < splits; ++s) v += p[s * len + i];
+    C[i] = v;
+  }
+}
+
+// The three-stage ring is above the 48 KB default; raised once per kernel and device.
+template <typename K>
+cudaError_t raise_shared(K kernel, bool (&raised)[64]) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= 64 || !raised[dev]) {
-    e = cudaFuncSetAttribute(dgemm_kernel<TA, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) raised[dev] = true;
   }
+  return cudaSuccess;
+}
+
+template <bool TA, bool TB>
+cudaError_t launch(cudaStream_t stream, const GemmArgs& g, dim3 grid) {
+  static bool raised[64] = {};
+  const cudaError_t e = raise_shared(dgemm_kernel<TA, TB>, raised);
+  if (e != cudaSuccess) return e;
   dgemm_kernel<TA, TB><<<grid, kThreads, kSmem, stream>>>(g);
+  return cudaGetLastError();
+}
+
+template <bool TA>
+cudaError_t launch_group(cudaStream_t stream, const GroupArgs& g, dim3 grid) {
+  static bool raised[64] = {};
+  const cudaError_t e = raise_shared(dgemm_group_kernel<TA>, raised);
+  if (e != cudaSuccess) return e;
+  dgemm_group_kernel<TA><<<grid, kThreads, kSmem, stream>>>(g);
   return cudaGetLastError();
 }
 
@@ -194,6 +253,53 @@ cudaError_t dgemm_strided(cudaStream_t stream, bool ta, bool tb, int M, int N, i
   const dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)batch);
   if (ta) return tb ? launch<true, true>(stream, g, grid) : launch<true, false>(stream, g, grid);
   return tb ? launch<false, true>(stream, g, grid) : launch<false, false>(stream, g, grid);
+}
+
+cudaError_t dgemm_group(cudaStream_t stream, bool ta, int n, const GemmGroup* entries, int count) {
+  while (count > 0) {
+    const int take = std::min(count, kGemmGroupMax);
+    GroupArgs g{};
+    g.n = n;
+    for (int i = 0; i < take; ++i) {
+      g.e[i] = entries[i];
+      g.most = std::max(g.most, entries[i].batch);
+    }
+    // grid.z holds at most 65535 products
+    const int fit = g.most > 0 ? std::max(1, std::min(take, 65535 / g.most)) : take;
+    if (g.most > 65535) return cudaErrorInvalidValue;
+    if (g.most > 0) {
+      const unsigned t = (unsigned)((n + kBM - 1) / kBM);
+      const dim3 grid(t, t, (unsigned)(fit * g.most));
+      const cudaError_t e = ta ? launch_group<true>(stream, g, grid) : launch_group<false>(stream, g, grid);
+      if (e != cudaSuccess) return e;
+    }
+    entries += fit;
+    count -= fit;
+  }
+  return cudaSuccess;
+}
+
+cudaError_t dgemm_nt_pair(cudaStream_t stream, int M, int N, int K, const double* A, const double* B0, double* C0,
+                          const double* B1, double* C1, double* scratch, size_t scratch_doubles) {
+  const long long gx = (N + kBN - 1) / kBN, gy = (M + kBM - 1) / kBM;
+  const int nk = (K + kBK - 1) / kBK;
+  const long long len = (long long)M * N;
+  // Three blocks fit an SM; split the reduction until two waves of them exist, eight panels a split at least.
+  long long want = (2 * 3 * 148 + 2 * gx * gy - 1) / (2 * gx * gy);
+  want = std::min<long long>(want, std::min<long long>(nk / 8, (long long)(scratch_doubles / (2 * (size_t)len))));
+  if (want < 2 || gy > 65535) {
+    const cudaError_t e = dgemm_strided(stream, false, true, M, N, K, 1.0, A, K, 0, B0, K, 0, 0.0, C0, N, 0, 1);
+    return e != cudaSuccess ? e : dgemm_strided(stream, false, true, M, N, K, 1.0, A, K, 0, B1, K, 0, 0.0, C1, N, 0, 1);
+  }
+  const int per = (int)((nk + want - 1) / want), splits = (nk + per - 1) / per;
+  static bool raised[64] = {};
+  const cudaError_t e = raise_shared(dgemm_split_kernel, raised);
+  if (e != cudaSuccess) return e;
+  const GemmArgs g{A, B0, scratch, 0, 0, len, M, N, K, K, K, N, 1.0, 0.0};
+  dgemm_split_kernel<<<dim3((unsigned)gx, (unsigned)gy, 2u * splits), kThreads, kSmem, stream>>>(g, B1, splits, per);
+  split_sum_kernel<<<dim3((unsigned)std::min<long long>((len + 255) / 256, 148 * 8), 2), 256, 0, stream>>>(scratch, splits, len,
+                                                                                                    C0, C1);
+  return cudaGetLastError();
 }
 
 }  // namespace nw

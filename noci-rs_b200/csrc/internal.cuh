@@ -200,6 +200,21 @@ cudaError_t dgemm_strided(cudaStream_t stream, bool ta, bool tb, int M, int N, i
                           int lda, long long sa, const double* B, int ldb, long long sb, double beta, double* C,
                           int ldc, long long sc, int batch);
 
+// Batches of row-major n x n products C[b] = op(A[b]) B[b] in one launch (op(A) = A^T with ta).
+constexpr int kGemmGroupMax = 32;
+struct GemmGroup {
+  const double* A;
+  const double* B;
+  double* C;
+  long long sa, sb, sc;   // batch strides (elements)
+  int batch;
+};
+cudaError_t dgemm_group(cudaStream_t stream, bool ta, int n, const GemmGroup* entries, int count);
+// C0 = A B0^T and C1 = A B1^T (A M x K, B0 and B1 N x K), the reduction split over blocks through `scratch`
+// and summed in a fixed order.
+cudaError_t dgemm_nt_pair(cudaStream_t stream, int M, int N, int K, const double* A, const double* B0, double* C0,
+                          const double* B1, double* C1, double* scratch, size_t scratch_doubles);
+
 // Cholesky-route product on tcgen05 (tc_gemm.cu): t4[p][r][q][s] = sum_k U[k][pq] V[k][rs] with
 // mode NW_TRANSFORM_CHOL_INT8 (8 int8 Ozaki slices) or NW_TRANSFORM_CHOL_BF16X6 (3 BF16 pieces).
 constexpr int kOzakiSlices = 8;
