@@ -108,6 +108,13 @@ cudaError_t pipe_drain(nw_ctx* ctx) {
   return first;
 }
 
+// Smallest chunk of the pipeline below.  With zero-overlap reference pairs a small chunk takes nearly as long
+// as a large one (n = 64: 65536 pairs 230 us, 300000 pairs 399 us), so those keep the large one.
+uint64_t pipe_min_chunk(nw_ctx* ctx, nw::EvalMode mode, uint64_t npairs) {
+  const bool gen = nw::any_generic(ctx);
+  return !gen && npairs <= nw::tile_limit(nw::make_params(ctx), mode, gen) ? nw::kPipeTileChunk : nw::kPipeMinChunk;
+}
+
 // Host-buffer evaluation as a three-stage pipeline over chunks of the request: chunk k+1 is
 // copied in (copy engine, host -> device) while chunk k is evaluated and chunk k-1 is copied
 // out (second copy engine, device -> host), so PCIe transfer in both directions overlaps the
@@ -123,7 +130,7 @@ nw_status eval_hs_pipelined(nw_ctx* ctx, nw::EvalMode mode, const uint32_t* pair
   for (cudaStream_t q : {ctx->s_in, ctx->s_comp, ctx->s_out}) NW_CUDA(ctx, cudaStreamWaitEvent(q, ctx->ev_start, 0));
   NW_CUDA(ctx, cudaMemsetAsync(flag, 0, sizeof(uint32_t), ctx->s_comp));
   uint64_t chunk = (npairs + nw::kPipeChunks - 1) / nw::kPipeChunks;
-  chunk = std::max<uint64_t>(nw::pipe_min_chunk(ctx), (chunk + 255) / 256 * 256);
+  chunk = std::max<uint64_t>(pipe_min_chunk(ctx, mode, npairs), (chunk + 255) / 256 * 256);
   uint64_t k = 0;
   for (uint64_t o = 0; o < npairs; o += chunk, ++k) {
     const uint64_t nk = std::min(chunk, npairs - o);
@@ -136,7 +143,7 @@ nw_status eval_hs_pipelined(nw_ctx* ctx, nw::EvalMode mode, const uint32_t* pair
       pipe_drain(ctx);
       return nw::cuda_fail(ctx, e, "pipelined copy-in");
     }
-    st = nw::eval_pairs(ctx, dp + 2 * o, nk, dh + 2 * o, mode, ctx->s_comp, false);
+    st = nw::eval_pairs(ctx, dp + 2 * o, nk, dh + 2 * o, mode, ctx->s_comp, false, npairs);
     if (st != NW_OK) {
       pipe_drain(ctx);
       return st;
@@ -171,7 +178,7 @@ nw_status eval_host(nw_ctx* ctx, nw::EvalMode mode, const uint32_t* pairs_host, 
   if ((st = nw::ensure(ctx, ctx->io_hs, npairs * 2 * sizeof(double))) != NW_OK) return st;
   uint32_t* dp = static_cast<uint32_t*>(ctx->io_pairs.p);
   double* dh = static_cast<double*>(ctx->io_hs.p);
-  if (npairs >= 2 * nw::pipe_min_chunk(ctx) && is_pinned(pairs_host) && is_pinned(out_host))
+  if (npairs >= 2 * pipe_min_chunk(ctx, mode, npairs) && is_pinned(pairs_host) && is_pinned(out_host))
     return eval_hs_pipelined(ctx, mode, pairs_host, npairs, out_host, dp, dh, s);
   NW_CUDA(ctx, cudaMemcpyAsync(dp, pairs_host, npairs * 2 * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
   if ((st = nw::eval_pairs(ctx, dp, npairs, dh, mode, s)) != NW_OK) return st;

@@ -624,11 +624,15 @@ nw_status launch_sorted(nw_ctx* ctx, const EvalParams& P, uint64_t nkeys, const 
 }
 
 
+bool any_generic(const nw_ctx* ctx) {
+  return std::find(ctx->generic_host.begin(), ctx->generic_host.end(), (char)1) != ctx->generic_host.end();
+}
+
 nw_status eval_pairs(nw_ctx* ctx, const uint32_t* pairs, uint64_t npairs, double* out, EvalMode mode,
-                     cudaStream_t stream, bool clear_flag) {
+                     cudaStream_t stream, bool clear_flag, uint64_t request) {
   if (!ctx->built) return fail(ctx, NW_ERR_STATE, "intermediates not built");
   if (!ctx->d_dets) return fail(ctx, NW_ERR_STATE, "no determinant basis set");
-  return eval_pairs_on(ctx, make_params(ctx), pairs, npairs, out, mode, stream, clear_flag);
+  return eval_pairs_on(ctx, make_params(ctx), pairs, npairs, out, mode, stream, clear_flag, request);
 }
 
 // Blocked evaluation for systems whose intermediates exceed the device memory: a build of no
@@ -696,7 +700,7 @@ nw_status eval_blocked(nw_ctx* ctx, const uint32_t* pairs, uint64_t npairs, doub
 }
 
 nw_status eval_pairs_on(nw_ctx* ctx, EvalParams P, const uint32_t* pairs, uint64_t npairs, double* out, EvalMode mode,
-                        cudaStream_t stream, bool clear_flag) {
+                        cudaStream_t stream, bool clear_flag, uint64_t request) {
   if (!ctx->built) return fail(ctx, NW_ERR_STATE, "intermediates not built");
   if (ctx->partial && !ctx->allow_partial)
     return fail(ctx, NW_ERR_STATE, "the intermediates hold one block of a blocked evaluation (rebuild them)");
@@ -719,8 +723,9 @@ nw_status eval_pairs_on(nw_ctx* ctx, EvalParams P, const uint32_t* pairs, uint64
     return NW_OK;
   }
 
-  const bool gen = ctx->nfast < ctx->nresident;
-  if (!(ctx->timing && ctx->serial_classes) && tile_route(P, npairs, mode, gen)) {
+  // the blocks of a blocked evaluation route like the full build
+  const bool gen = any_generic(ctx);
+  if (!(ctx->timing && ctx->serial_classes) && std::max(npairs, request) <= tile_limit(P, mode, gen)) {
     // phase events: everything is the evaluator's
     if (ctx->timing)
       for (int i = 0; i < 4; ++i) NW_CUDA(ctx, cudaEventRecord(ctx->ev[i], stream));

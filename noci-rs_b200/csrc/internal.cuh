@@ -175,11 +175,11 @@ struct CtxGuard {
 };
 
 
-// Pipelined host-buffer path: about kPipeChunks chunks of at least pipe_min_chunk pairs.  A chunk of 65536
-// takes one evaluation launch (17 us at n = 30) beside the 20 us of its copy out; with zero-overlap reference
-// pairs a chunk of that size takes 230 us against 399 us for 300000 pairs at once, so those stay at 2^18.
+// Pipelined host-buffer path: about kPipeChunks chunks of at least kPipeMinChunk pairs, or of kPipeTileChunk
+// where one launch evaluates a chunk (17 us at n = 30 beside the 20 us of its copy out).
 constexpr uint64_t kPipeChunks = 16;
-inline uint64_t pipe_min_chunk(const nw_ctx* ctx) { return ctx->nfast < ctx->nresident ? 1ull << 18 : 1ull << 16; }
+constexpr uint64_t kPipeMinChunk = 1ull << 18;
+constexpr uint64_t kPipeTileChunk = 1ull << 16;
 
 // Records an error on the context and returns the status.
 nw_status fail(nw_ctx* ctx, nw_status st, const std::string& msg);
@@ -280,13 +280,17 @@ nw_status update_fock(nw_ctx* ctx, const double* fa, const double* fb);
 enum class EvalMode { kHS, kS, kFS };
 
 // Evaluation (eval.cu).
-// clear_flag = false keeps the out-of-range flag of earlier calls (chunked host path).
+// clear_flag = false keeps the out-of-range flag of earlier calls (chunked host path); `request` is the
+// size of the whole request where this call evaluates a chunk of it (the route, and with it the last bit
+// of an element, is the whole request's).
 nw_status eval_pairs(nw_ctx* ctx, const uint32_t* pairs, uint64_t npairs, double* out, EvalMode mode,
-                     cudaStream_t stream, bool clear_flag = true);
+                     cudaStream_t stream, bool clear_flag = true, uint64_t request = 0);
+// Some reference pair has zero-overlap orbitals, resident or not.
+bool any_generic(const nw_ctx* ctx);
 // The same over a caller-supplied determinant table (P.dets / P.desc / P.ndet), e.g. the records
 // packed from excitation caches by nw_eval_hs_batched.
 nw_status eval_pairs_on(nw_ctx* ctx, EvalParams P, const uint32_t* pairs, uint64_t npairs, double* out, EvalMode mode,
-                        cudaStream_t stream, bool clear_flag = true);
+                        cudaStream_t stream, bool clear_flag = true, uint64_t request = 0);
 // Dense matrices over left x right determinant blocks and the generalised eigenproblem (matrix.cu).
 nw_status build_matrix(nw_ctx* ctx, EvalMode mode, const uint32_t* left, uint64_t nl, const uint32_t* right,
                        uint64_t nr, bool symmetric, double* a_host, double* s_host);
@@ -310,12 +314,14 @@ struct SortScratch {
 constexpr uint64_t kFineMax = 1ull << 23;
 constexpr uint64_t kFineMin = 1ull << 14;
 // Largest requests that take the one-kernel evaluation (tile_eval.cu) where the sorted pipeline's order
-// pays for larger ones.  Measured, sorted / one kernel, us: (H, S) at n = 30, 3 references: 512 pairs
-// 37.7 / 10.3, 131072 pairs 51 / 25, 10^6 pairs 109 / 152; n = 64, 6 references: 131072 pairs 76 / 72,
-// 300000 pairs 103 / 153; n = 64 with zero-overlap reference pairs: 131072 pairs 357 / 286, 300000
-// pairs 399 / 574.
-constexpr uint64_t kTileSmallHS = 1ull << 17;
-constexpr uint64_t kTileSmallFS = 1ull << 17;
+// pays for larger ones: kTileLarge while the n^4 tables of one reference pair (three of 8 n^4 bytes) fit in
+// half of L2, else kTileSmall.  Measured, sorted / one kernel, us: (H, S) at n = 30, 3 references: 512 pairs
+// 37.7 / 10.3, 131072 pairs 51 / 25, 300000 pairs 61 / 47, 10^6 pairs 109 / 152; n = 40: 300000 pairs
+// 69 / 51, 10^6 pairs 127 / 164; n = 64, 6 references: 131072 pairs 76 / 72, 300000 pairs 103 / 153; n = 64
+// with zero-overlap reference pairs: 131072 pairs 357 / 286, 300000 pairs 399 / 574.
+constexpr uint64_t kTileSmall = 1ull << 17;
+constexpr uint64_t kTileLarge = 3ull << 17;
+constexpr uint64_t kTileTables = 64ull << 20;
 
 EvalParams make_params(const nw_ctx* ctx);
 // Number of sort keys with at most `cap` counters for the fast classes and at most gen_cap for the
@@ -331,9 +337,9 @@ nw_status launch_sorted(nw_ctx* ctx, const EvalParams& P, uint64_t nkeys, const 
                         EvalMode mode = EvalMode::kHS, const uint32_t* npairs_dev = nullptr,
                         bool classified = false);
 
-// One-kernel evaluation of a request (tile_eval.cu): whether `npairs` pairs take it (gen: some resident
+// One-kernel evaluation of a request (tile_eval.cu): the largest request that takes it (gen: some
 // reference pair has zero-overlap orbitals), and the launch.
-bool tile_route(const EvalParams& P, uint64_t npairs, EvalMode mode, bool gen);
+uint64_t tile_limit(const EvalParams& P, EvalMode mode, bool gen);
 cudaError_t eval_tiles(const EvalParams& P, const uint2* pairs, uint64_t npairs, double* out, EvalMode mode, bool gen,
                        uint32_t* flag, cudaStream_t stream);
 

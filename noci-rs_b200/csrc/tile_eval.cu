@@ -267,10 +267,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) hs_tile_kernel(EvalParams P, 
 
 }  // namespace
 
-// (F, S) without zero-overlap reference pairs always, other requests up to the sizes at kTileSmallHS.
-bool tile_route(const EvalParams& P, uint64_t npairs, EvalMode mode, bool gen) {
-  if (mode == EvalMode::kFS) return !gen || npairs <= kTileSmallFS;
-  return npairs <= kTileSmallHS;
+uint64_t tile_limit(const EvalParams& P, EvalMode mode, bool gen) {
+  if (mode == EvalMode::kFS) return gen ? kTileSmall : ~0ull;
+  return !gen && (uint64_t)P.n * P.n * P.n * P.n * 24 <= kTileTables ? kTileLarge : kTileSmall;
 }
 
 cudaError_t eval_tiles(const EvalParams& P, const uint2* pairs, uint64_t npairs, double* out, EvalMode mode, bool gen,

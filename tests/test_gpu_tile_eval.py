@@ -50,7 +50,7 @@ def test_routes_agree(zero_pairs, fs):
     with nociwick.WicksShared(system.s, system.h, system.eri, system.enuc, system.refs, tol=1e-8) as w:
         w.build().set_basis(basis)
         w.update_fock(*fock)
-        for n in (1, 31, 33, 148 * 32 + 1, 20000, 131072, 131073, 148 * 1024 + 7):
+        for n in (1, 31, 33, 148 * 32 + 1, 20000, 131072, 131073, 148 * 1024 + 7, 393216, 393217):
             pairs = sy.sample_pairs(basis, n, seed=n, distinct_parents=False)
             one, srt = _both(w, torch, pairs, fs)
             assert np.all(np.isfinite(one)) and np.max(np.abs(one - srt)) <= ROUTES, n
@@ -95,7 +95,7 @@ def test_pinned_host_chunks(zero_pairs):
     basis = sy.sd_basis(10, 3, 3, 3)
     with nociwick.WicksShared(system.s, system.h, system.eri, system.enuc, system.refs, tol=1e-8) as w:
         w.build().set_basis(basis)
-        for n in ((1 << 17) - 1, 1 << 17, 200_001, 600_001):
+        for n in ((1 << 17) - 1, 1 << 17, 200_001, 393_216, 393_217, 600_001):
             pairs = sy.sample_pairs(basis, n, seed=n, distinct_parents=False)
             host = torch.from_numpy(pairs.astype(np.uint32).view(np.int32)).pin_memory()
             out = torch.full((n, 2), float("nan"), dtype=torch.float64).pin_memory()
