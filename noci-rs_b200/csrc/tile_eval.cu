@@ -5,9 +5,10 @@
 // memory: five passes over 4-byte keys, ranks and indices and twelve dependent launches, so that the
 // n^4 tables are read with locality.  Two kinds of request do not need that order:
 //  * (F, S): the tables of one reference pair are four n^2 record arrays (100 KB at n = 40), L1 / L2
-//    resident however the pairs come.  4 10^6 pairs at n = 28 (9 + 9 electrons, 3 references): 270 us
-//    sorted, 233 us here (L1 gathers at 74 % of the L1TEX limit, 24 warps per SM; 1000 pairs 31 -> 8.3 us);
-//    n = 40, 8 references, ranks 0-4: 292 -> 215 us.
+//    resident however the pairs come.  4 10^6 pairs at n = 28 (9 + 9 electrons, 3 references): 276 us
+//    sorted, 207 us here (L1 gathers at 76 % of the L1TEX limit, hit rate 45 %, 24 warps per SM; 1000 pairs
+//    31 -> 8.3 us); n = 40, 6 + 6 electrons, ranks 0-4: 158 us.  Reading the factors of single-single string
+//    pairs from a table of all of them instead of the records was slower (252 us).
 //  * small (H, S) requests: the chain of launches is longer than the work (512 pairs at n = 30: 37.7 ->
 //    10.3 us).
 // A tile of 1024 pairs holds some ten classes, so whole-warp padding costs about a sixth of the lanes.
@@ -57,7 +58,7 @@ __device__ __forceinline__ int tile_classify(const EvalParams& P, uint2 ab, uint
   return c;
 }
 
-// Groups the block's tile [base, base + count) by class and calls eval(class, request index, bra, ket)
+// Groups the block's tile [base, base + count) by class and calls eval(class, request index, pair)
 // for every pair to evaluate; the lanes of a warp always hold one class.  Chunks of 32 slots go to the
 // warps from the last class down, so the ranks with the most work start first.
 template <bool GEN, typename F>
@@ -132,7 +133,7 @@ __device__ __forceinline__ void tile_run(const EvalParams& P, const uint2* __res
     const uint32_t k = s_slot[slot0 + lane];
     if (k != 0xFFFFu) {
       const uint2 ab = s_ab[k];
-      eval(c, base + k, load_det(P.dets, ab.x), load_det(P.dets, ab.y));
+      eval(c, base + k, ab);
     }
     __syncwarp();
   }
@@ -171,23 +172,28 @@ __device__ __forceinline__ void spin_f_of(int L, const double2* __restrict__ rec
   }
 }
 
-__device__ __noinline__ void fs_rt_one(const FastPair& fp, const FockPair& fk, const DetRec& x, const DetRec& w, int n,
-                                       int oa, int ob, double* f, double* s) {
-  eval_fs_m0_rt(fp, fk, x, w, n, oa, ob, f, s);
+// The rare paths are calls that take everything by value and load the records themselves: a reference to a
+// record or to the kernel's parameters would keep them in local memory on the common path too (4 10^6 (F, S)
+// pairs: 235 us with references, 207 us without).
+__device__ __noinline__ double2 fs_rt_one(const EvalParams* P, uint2 ab) {
+  const DetRec x = load_det(P->dets, ab.x), w = load_det(P->dets, ab.y);
+  const int p = (int)x.parent * P->nref + (int)w.parent;
+  double2 r;
+  eval_fs_m0_rt(P->fast[p], P->fock[p], x, w, P->n, P->nocc_a, P->nocc_b, &r.x, &r.y);
+  return r;
 }
 
-__device__ __noinline__ void fs_gen_one(const GenPair& g, const FockPair& fk, const DetRec& x, const DetRec& w,
-                                        const EvalParams& P, double* f, double* s) {
-  eval_fs_gen_any(g, fk, x, w, P.n, P.nocc_a, P.nocc_b, P.tol, P.exact != 0, f, s);
+__device__ __noinline__ double2 fs_gen_one(const EvalParams* P, uint2 ab) {
+  const DetRec x = load_det(P->dets, ab.x), w = load_det(P->dets, ab.y);
+  const int p = (int)x.parent * P->nref + (int)w.parent;
+  double2 r;
+  eval_fs_gen_any(P->gen[p], P->fock[p], x, w, P->n, P->nocc_a, P->nocc_b, P->tol, P->exact != 0, &r.x, &r.y);
+  return r;
 }
 
-__device__ __forceinline__ void fs_fast(const EvalParams& P, int c, const DetRec& x, const DetRec& w, double* f,
-                                        double* s) {
+__device__ __forceinline__ void fs_fast(const EvalParams& P, int c, uint2 ab, double* f, double* s) {
+  const DetRec x = load_det(P.dets, ab.x), w = load_det(P.dets, ab.y);
   const int p = (int)x.parent * P.nref + (int)w.parent;
-  if (c == kClasses - 1) {
-    fs_rt_one(P.fast[p], P.fock[p], x, w, P.n, P.nocc_a, P.nocc_b, f, s);
-    return;
-  }
   // the slab of the Fock records is regular: recx, recy of alpha, then of beta, per ordered pair
   const int la = c / 5, lb = c - 5 * la, n2 = P.n * P.n;
   const double* rec = P.fslab + (size_t)p * (8 * n2);
@@ -201,35 +207,40 @@ __device__ __forceinline__ void fs_fast(const EvalParams& P, int c, const DetRec
 }
 
 template <bool GEN, int MINB>
-__global__ void __launch_bounds__(kTileThreads, MINB) fs_tile_kernel(EvalParams P, const uint2* __restrict__ pairs,
+__global__ void __launch_bounds__(kTileThreads, MINB) fs_tile_kernel(const __grid_constant__ EvalParams P, const uint2* __restrict__ pairs,
                                                                      uint64_t npairs, int tile,
                                                                      double* __restrict__ out,
                                                                      uint32_t* __restrict__ flag) {
   const uint64_t base = (uint64_t)blockIdx.x * (uint64_t)tile;
   const int count = (int)min((uint64_t)tile, npairs - base);
-  tile_run<GEN>(P, pairs, base, count, out, flag, [&](int c, uint64_t i, const DetRec& x, const DetRec& w) {
-    double f, s;
-    if (GEN && c >= kClasses) {
-      const int p = (int)x.parent * P.nref + (int)w.parent;
-      fs_gen_one(P.gen[p], P.fock[p], x, w, P, &f, &s);
-    } else {
-      fs_fast(P, c, x, w, &f, &s);
-    }
-    store_hs(out, i, f, s);
+  tile_run<GEN>(P, pairs, base, count, out, flag, [&](int c, uint64_t i, uint2 ab) {
+    double2 r;
+    if (GEN && c >= kClasses)
+      r = fs_gen_one(&P, ab);
+    else if (c == kClasses - 1)
+      r = fs_rt_one(&P, ab);
+    else
+      fs_fast(P, c, ab, &r.x, &r.y);
+    store_hs(out, i, r.x, r.y);
   });
 }
 
 // ---------------------------------------------------------------------------------------
 // (H, S) of small requests.
 // ---------------------------------------------------------------------------------------
-__device__ __noinline__ void hs_rt_one(const FastPair& fp, const DetRec& x, const DetRec& w, const EvalParams& P,
-                                       double* h, double* s) {
-  eval_m0_rt(fp, x, w, P.n, P.nocc_a, P.nocc_b, P.enuc, h, s);
+__device__ __noinline__ double2 hs_rt_one(const EvalParams* P, uint2 ab) {
+  const DetRec x = load_det(P->dets, ab.x), w = load_det(P->dets, ab.y);
+  double2 r;
+  eval_m0_rt(P->fast[(int)x.parent * P->nref + (int)w.parent], x, w, P->n, P->nocc_a, P->nocc_b, P->enuc, &r.x, &r.y);
+  return r;
 }
 
-__device__ __noinline__ void hs_gen_one(const GenPair& g, const DetRec& x, const DetRec& w, const EvalParams& P, double* h,
-                                        double* s) {
-  eval_gen_any(g, x, w, P.n, P.nocc_a, P.nocc_b, P.enuc, P.tol, P.exact != 0, h, s);
+__device__ __noinline__ double2 hs_gen_one(const EvalParams* P, uint2 ab) {
+  const DetRec x = load_det(P->dets, ab.x), w = load_det(P->dets, ab.y);
+  double2 r;
+  eval_gen_any(P->gen[(int)x.parent * P->nref + (int)w.parent], x, w, P->n, P->nocc_a, P->nocc_b, P->enuc, P->tol,
+               P->exact != 0, &r.x, &r.y);
+  return r;
 }
 
 #define NW_HS_TILE_CASE(A, B)                                                       \
@@ -238,27 +249,31 @@ __device__ __noinline__ void hs_gen_one(const GenPair& g, const DetRec& x, const
     break;
 
 template <bool GEN>
-__global__ void __launch_bounds__(kTileThreads, 1) hs_tile_kernel(EvalParams P, const uint2* __restrict__ pairs,
+__global__ void __launch_bounds__(kTileThreads, 1) hs_tile_kernel(const __grid_constant__ EvalParams P, const uint2* __restrict__ pairs,
                                                                uint64_t npairs, int tile, double* __restrict__ out,
                                                                uint32_t* __restrict__ flag) {
   const uint64_t base = (uint64_t)blockIdx.x * (uint64_t)tile;
   const int count = (int)min((uint64_t)tile, npairs - base);
-  tile_run<GEN>(P, pairs, base, count, out, flag, [&](int c, uint64_t i, const DetRec& x, const DetRec& w) {
-    const int p = (int)x.parent * P.nref + (int)w.parent;
-    double h, s;
+  tile_run<GEN>(P, pairs, base, count, out, flag, [&](int c, uint64_t i, uint2 ab) {
     if (GEN && c >= kClasses) {
-      hs_gen_one(P.gen[p], x, w, P, &h, &s);
-    } else {
-      switch (c) {
-        NW_HS_TILE_CASE(0, 0) NW_HS_TILE_CASE(0, 1) NW_HS_TILE_CASE(0, 2) NW_HS_TILE_CASE(0, 3) NW_HS_TILE_CASE(0, 4)
-        NW_HS_TILE_CASE(1, 0) NW_HS_TILE_CASE(1, 1) NW_HS_TILE_CASE(1, 2) NW_HS_TILE_CASE(1, 3) NW_HS_TILE_CASE(1, 4)
-        NW_HS_TILE_CASE(2, 0) NW_HS_TILE_CASE(2, 1) NW_HS_TILE_CASE(2, 2) NW_HS_TILE_CASE(2, 3) NW_HS_TILE_CASE(2, 4)
-        NW_HS_TILE_CASE(3, 0) NW_HS_TILE_CASE(3, 1) NW_HS_TILE_CASE(3, 2) NW_HS_TILE_CASE(3, 3) NW_HS_TILE_CASE(3, 4)
-        NW_HS_TILE_CASE(4, 0) NW_HS_TILE_CASE(4, 1) NW_HS_TILE_CASE(4, 2) NW_HS_TILE_CASE(4, 3) NW_HS_TILE_CASE(4, 4)
-        default:
-          hs_rt_one(P.fast[p], x, w, P, &h, &s);
-          break;
-      }
+      const double2 r = hs_gen_one(&P, ab);
+      store_hs(out, i, r.x, r.y);
+      return;
+    }
+    if (c == kClasses - 1) {
+      const double2 r = hs_rt_one(&P, ab);
+      store_hs(out, i, r.x, r.y);
+      return;
+    }
+    const DetRec x = load_det(P.dets, ab.x), w = load_det(P.dets, ab.y);
+    const int p = (int)x.parent * P.nref + (int)w.parent;
+    double h = 0.0, s = 0.0;
+    switch (c) {
+      NW_HS_TILE_CASE(0, 0) NW_HS_TILE_CASE(0, 1) NW_HS_TILE_CASE(0, 2) NW_HS_TILE_CASE(0, 3) NW_HS_TILE_CASE(0, 4)
+      NW_HS_TILE_CASE(1, 0) NW_HS_TILE_CASE(1, 1) NW_HS_TILE_CASE(1, 2) NW_HS_TILE_CASE(1, 3) NW_HS_TILE_CASE(1, 4)
+      NW_HS_TILE_CASE(2, 0) NW_HS_TILE_CASE(2, 1) NW_HS_TILE_CASE(2, 2) NW_HS_TILE_CASE(2, 3) NW_HS_TILE_CASE(2, 4)
+      NW_HS_TILE_CASE(3, 0) NW_HS_TILE_CASE(3, 1) NW_HS_TILE_CASE(3, 2) NW_HS_TILE_CASE(3, 3) NW_HS_TILE_CASE(3, 4)
+      NW_HS_TILE_CASE(4, 0) NW_HS_TILE_CASE(4, 1) NW_HS_TILE_CASE(4, 2) NW_HS_TILE_CASE(4, 3) NW_HS_TILE_CASE(4, 4)
     }
     store_hs(out, i, h, s);
   });
