@@ -20,7 +20,8 @@
 //
 // Measured (B200): the second half at n = 64 runs at 28 TFLOP/s (FP64 tensor pipe 79 % active, ncu), the
 // quarter transforms at 21; a build of 3 references with one zero-overlap reference pair, 31.7 -> 12.5 ms
-// at n = 64 and, without one, 3.36 -> 0.91 ms at n = 30.  Larger n (matrices beyond shared memory) and tensors
+// at n = 64 and, without one, 3.36 -> 0.91 ms at n = 30 (11.2 and 0.475 ms since the other products of the build
+// share launches).  Larger n (matrices beyond shared memory) and tensors
 // without the symmetry keep the quarter transforms.
 #include <cuda_runtime.h>
 
