@@ -25,10 +25,13 @@ nw_status cuda_fail(nw_ctx* ctx, cudaError_t e, const char* what) {
 
 cudaError_t ctx_malloc(nw_ctx* ctx, void** p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, bytes);
-  if (e == cudaErrorMemoryAllocation && ctx->pt2_spare.p) {
+  if (e != cudaErrorMemoryAllocation) return e;
+  std::lock_guard<std::mutex> lock(ctx->pt2_spare->mtx);
+  DevBuf& spare = ctx->pt2_spare->buf;
+  if (spare.p) {
     cudaGetLastError();
-    cudaFree(ctx->pt2_spare.p);
-    ctx->pt2_spare = DevBuf{};
+    cudaFree(spare.p);
+    spare = DevBuf{};
     e = cudaMalloc(p, bytes);
   }
   return e;
@@ -595,7 +598,11 @@ nw_status nw_ctx_destroy(nw_ctx* ctx) {
   free_buf(ctx->build_tasks);
   free_buf(ctx->pt2_scratch);
   free_buf(ctx->pt2_table);
-  free_buf(ctx->pt2_spare);
+  {
+    std::lock_guard<std::mutex> lock(ctx->pt2_spare->mtx);
+    free_buf(ctx->pt2_spare->buf);
+    ctx->pt2_spare->open = false;
+  }
   free_buf(ctx->gmres_work);
   free_buf(ctx->bt_dets);
   free_buf(ctx->bt_desc);

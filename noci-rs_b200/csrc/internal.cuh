@@ -7,6 +7,7 @@
 #include <cusolverDn.h>
 #include <stdint.h>
 
+#include <memory>
 #include <mutex>
 
 #include <string>
@@ -46,6 +47,14 @@ struct EvalParams {
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
+};
+
+// The matrix of the last destroyed candidate operator (at most kKeepMatrix bytes), shared with the
+// operators of a context: one that outlives its context finds it closed.
+struct SpareMatrix {
+  std::mutex mtx;
+  bool open = true;
+  DevBuf buf;
 };
 
 // Spin-factorised overlap action over the resident basis (overlap.cu).
@@ -96,7 +105,7 @@ struct nw_ctx {
 
   // packed candidate matrix: strings of the candidates, and their pair tables (pt2_strings.cu)
   nw::DevBuf pt2_scratch, pt2_table;
-  nw::DevBuf pt2_spare;            // matrix of the last destroyed operator (at most kKeepMatrix bytes)
+  std::shared_ptr<nw::SpareMatrix> pt2_spare = std::make_shared<nw::SpareMatrix>();
   nw::DevBuf gmres_work;           // vectors and scratch of the solves (kept up to kKeepGmres bytes)
 
   // evaluation scratch (grown on demand)

@@ -32,6 +32,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstddef>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <string>
@@ -525,6 +526,8 @@ __global__ void arn_init_kernel(ArnoldiState* __restrict__ st, int inner, double
 
 struct nw_pt2 {
   nw_ctx* ctx = nullptr;
+  int device = 0;
+  std::shared_ptr<nw::SpareMatrix> spare;
   uint64_t n = 0;
   double e0 = 0.0;
   double* m = nullptr;      // packed upper triangle, n (n + 1) / 2 (null when matrix-free)
@@ -637,6 +640,8 @@ nw_status nw_pt2_create(nw_ctx* ctx, const uint32_t* cand, uint64_t n, double e0
   nw_pt2* p = new (std::nothrow) nw_pt2;
   if (!p) return NW_ERR_ALLOC;
   p->ctx = ctx;
+  p->device = ctx->device;
+  p->spare = ctx->pt2_spare;
   p->n = n;
   p->e0 = e0;
   const uint64_t len = n * (n + 1) / 2;
@@ -656,11 +661,16 @@ nw_status nw_pt2_create(nw_ctx* ctx, const uint32_t* cand, uint64_t n, double e0
   };
   // the spare matrix of the context, unless much of it would lie idle
   p->m_bytes = sizeof(double) * len;
-  if (ctx->pt2_spare.bytes >= p->m_bytes && ctx->pt2_spare.bytes / 4 <= p->m_bytes) {
-    p->m = static_cast<double*>(ctx->pt2_spare.p);
-    p->m_bytes = ctx->pt2_spare.bytes;
-    ctx->pt2_spare = nw::DevBuf{};
-  } else if (nw::ctx_malloc(ctx, reinterpret_cast<void**>(&p->m), p->m_bytes) != cudaSuccess) {
+  {
+    std::lock_guard<std::mutex> lock(ctx->pt2_spare->mtx);
+    nw::DevBuf& spare = ctx->pt2_spare->buf;
+    if (spare.bytes >= p->m_bytes && spare.bytes / 4 <= p->m_bytes) {
+      p->m = static_cast<double*>(spare.p);
+      p->m_bytes = spare.bytes;
+      spare = nw::DevBuf{};
+    }
+  }
+  if (!p->m && nw::ctx_malloc(ctx, reinterpret_cast<void**>(&p->m), p->m_bytes) != cudaSuccess) {
     p->m = nullptr;
   }
   if (!p->m || nw::ctx_malloc(ctx, reinterpret_cast<void**>(&p->mdiag), sizeof(double) * 3 * n) != cudaSuccess)
@@ -707,6 +717,8 @@ nw_status nw_pt2_create_matrix_free(nw_ctx* ctx, const uint32_t* cand, uint64_t 
   nw_pt2* p = new (std::nothrow) nw_pt2;
   if (!p) return NW_ERR_ALLOC;
   p->ctx = ctx;
+  p->device = ctx->device;
+  p->spare = ctx->pt2_spare;
   p->n = n;
   p->e0 = e0;
   // pairs per evaluation block: 2^26 (1.6 GB of pairs and (F, S)) keeps the per-block cost of
@@ -980,13 +992,13 @@ nw_status nw_pt2_solve(nw_pt2* p, const nw_pt2_projection* proj, const double* r
 
 nw_status nw_pt2_destroy(nw_pt2* p) {
   if (!p) return NW_OK;
-  cudaSetDevice(p->ctx->device);
+  cudaSetDevice(p->device);
   cudaDeviceSynchronize();
   if (p->m && p->m_bytes <= nw::kKeepMatrix) {
     // the larger of this matrix and the spare one stays with the context
-    std::lock_guard<std::recursive_mutex> lock(p->ctx->mtx);
-    nw::DevBuf& spare = p->ctx->pt2_spare;
-    if (p->m_bytes > spare.bytes) {
+    std::lock_guard<std::mutex> lock(p->spare->mtx);
+    nw::DevBuf& spare = p->spare->buf;
+    if (p->spare->open && p->m_bytes > spare.bytes) {
       if (spare.p) cudaFree(spare.p);
       spare.p = p->m;
       spare.bytes = p->m_bytes;

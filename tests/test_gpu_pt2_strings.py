@@ -101,3 +101,15 @@ def test_matrix_and_vectors_kept_between_operators():
                 assert gi["iterations"] == si["iterations"]
                 assert np.max(np.abs(gx - sx)) <= 1e-6 * max(1.0, np.max(np.abs(sx)))
                 assert np.max(np.abs(other.apply_m(xs[1]) - fresh[1])) <= 1e-11 * max(1.0, np.max(np.abs(fresh[1])))
+
+
+def test_operator_outlives_its_context():
+    """An operator destroyed after its context gives its matrix back to the device, not to the context."""
+    system = sy.make_system(10, 3, 3, 3, 24, seed=7, k_scale=0.3)
+    basis = sy.sd_basis(10, 3, 3, 3)
+    w = nociwick.WicksShared(system.s, system.h, system.eri, system.enuc, system.refs, tol=1e-8)
+    w.build().set_basis(basis)
+    w.update_fock(system.h, system.h)
+    pt = nociwick.Pt2(w, np.arange(1200, dtype=np.uint32), -0.5)
+    w.close()
+    pt.close()
