@@ -523,8 +523,10 @@ nw_status upload_tasks(nw_ctx* ctx, const std::vector<T>& v, T** out) {
 // The fused route: J and II of every resident pair.  Without zero-overlap orbitals the intermediates
 // of (w, x) are those of (x, w) with rows and columns exchanged (M -> M^T), so only x <= w is
 // transformed and the other is a permuted copy; and the exchange part of the antisymmetrised J cancels
-// (it is symmetric in the columns that are exchanged), leaving N[ab|cd] - N[ad|cb].  `plan` holds
-// the tensors of the pairs with zero-overlap orbitals.
+// (it is symmetric in the columns that are exchanged), leaving N[ab|cd] - N[ad|cb].  The two orders of a
+// pair are decomposed separately, so a singular value within rounding of the tolerance can be zero in one
+// order only: the other order is then transformed itself.  `plan` holds the tensors of the pairs with
+// zero-overlap orbitals.
 template <typename Res, typename F1, typename F2>
 nw_status run_fused(nw_ctx* ctx, FusedPlan& plan, int n, int nref, const Res& resident, const std::vector<char>& generic,
                     const std::vector<FastOff>& fo, const F1& CX, const F2& XC, double* S0, double* work, size_t cap) {
@@ -542,7 +544,7 @@ nw_status run_fused(nw_ctx* ctx, FusedPlan& plan, int n, int nref, const Res& re
     for (int w = 0; w < nref; ++w) {
       const int p = x * nref + w, q = w * nref + x;
       if (!resident(p) || generic[p]) continue;
-      if (x > w) {
+      if (x > w && !generic[q]) {
         if (!resident(q)) {
           orphans.push_back(p);
           continue;

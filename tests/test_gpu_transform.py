@@ -53,3 +53,47 @@ def test_tensor_without_permutation_symmetry():
     basis = sy.sd_basis(12, 2, 3, 3)
     pairs = sy.sample_pairs(basis, 3000, seed=5, distinct_parents=True, canonical=False)
     _check(system, basis, pairs, convention="reference")
+
+
+def _split_classes():
+    """A system and a tolerance between the singular values that the two orders of one reference pair
+    compute for the same orbital pair: (1, 0) has no zero-overlap orbital and (0, 1) has one."""
+    for seed in range(60):
+        system = sy.make_system(10, 3, 3, 2, 24, seed=seed, k_scale=0.3, enuc=0.2)
+        (xa, _, xb, _), (wa, _, wb, _) = system.refs
+        s = min(np.linalg.svd(x[:, :3].T @ w[:, :3], compute_uv=False)[-1] for x, w in ((xa, wa), (xb, wb)))
+        if s < 0.2:
+            continue
+        for k in range(-12, 13):
+            tol = float(s + k * np.spacing(s))
+            with nociwick.WicksShared(system.s, system.h, system.eri, system.enuc, system.refs, tol=tol).build() as w:
+                m = w.zero_counts().sum(axis=2)
+            if (m[1, 0] == 0) != (m[0, 1] == 0):
+                if m[1, 0] > 0:
+                    system.refs.reverse()
+                return system, tol
+    raise AssertionError("no pair whose two orders round apart")
+
+
+def test_orders_of_a_pair_classed_apart():
+    """The order without zero-overlap orbitals keeps its own tensors where the other order has some: its
+    elements are the exact ones, in a full build and in every block of a blocked evaluation."""
+    import torch
+    system, tol = _split_classes()
+    basis = sy.sd_basis(10, 3, 3, 2)
+    per = basis.shape[0] // 2
+    rng = np.random.default_rng(2)
+    pairs = np.stack([per + rng.integers(0, per, 3000), rng.integers(0, per, 3000)], axis=1).astype(np.uint32)
+    orc = Oracle.from_system(system, tol=1e-8, with_mo_cache=False)
+    h, s = orc.eval_pairs(orc.oracle_basis(basis), pairs)
+    with nociwick.WicksShared(system.s, system.h, system.eri, system.enuc, system.refs, tol=tol).build() as w:
+        w.set_basis(basis)
+        hs = w.eval_pairs(pairs)
+        slab = w.info()["slab_bytes"]
+        assert np.max(np.abs(hs[:, 0] - h)) <= ATOL and np.max(np.abs(hs[:, 1] - s)) <= ATOL
+        stream = torch.cuda.current_stream().cuda_stream
+        dp = torch.from_numpy(pairs.view(np.int32)).cuda()
+        out = torch.full((pairs.shape[0], 2), float("nan"), dtype=torch.float64, device="cuda")
+        assert w.eval_pairs_blocked(dp.data_ptr(), pairs.shape[0], out.data_ptr(), slab // 2, stream) >= 2
+        torch.cuda.synchronize()
+        assert np.array_equal(out.cpu().numpy(), hs)
