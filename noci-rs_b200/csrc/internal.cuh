@@ -322,15 +322,24 @@ struct SortScratch {
 // per pair of the request so the counter memset and scan stay small next to the evaluation.
 constexpr uint64_t kFineMax = 1ull << 23;
 constexpr uint64_t kFineMin = 1ull << 14;
-// Largest requests that take the one-kernel evaluation (tile_eval.cu) where the sorted pipeline's order
-// pays for larger ones: kTileLarge while the n^4 tables of one reference pair (three of 8 n^4 bytes) fit in
-// half of L2, else kTileSmall.  Measured, sorted / one kernel, us: (H, S) at n = 30, 3 references: 512 pairs
-// 37.7 / 10.3, 131072 pairs 51 / 25, 300000 pairs 61 / 47, 10^6 pairs 109 / 152; n = 40: 300000 pairs
-// 69 / 51, 10^6 pairs 127 / 164; n = 64, 6 references: 131072 pairs 76 / 72, 300000 pairs 103 / 153; n = 64
-// with zero-overlap reference pairs: 131072 pairs 357 / 286, 300000 pairs 399 / 574.
-constexpr uint64_t kTileSmall = 1ull << 17;
+// Largest (H, S) requests that take the one-kernel evaluation (tile_eval.cu); the sorted pipeline's order pays
+// for larger ones.  A tile of unordered pairs reads the tables of every reference pair, so the line falls as
+// references are added; between 12 and 40 orbitals it follows nref^2 n^3 (singles and doubles, 2 to 48
+// references).  Time of the sorted pipeline over the one kernel's, for uniform pairs of all references and of
+// different ones / for pairs whose total rank is uniform over 0..4:
+//   nref^2 n^3 <= 10^6 (3 references to n = 40, 5 at n = 30, 8 at n = 24, 24 at n = 12)
+//       300000 pairs 0.94 to 1.74 (one kernel: two waves of tiles), 350000 pairs 0.82 to 1.26;
+//       up to 3 references 393216 pairs 1.06 to 1.38 / 1.5
+//   beyond
+//       65536 pairs 1.1 to 2.3 / 2.2 to 2.8, 131072 pairs 0.79 to 1.5 / 1.5 to 2.0,
+//       200000 pairs 0.55 to 1.05 / 1.1 to 1.4, 300000 pairs 0.49 to 0.91 / 0.92 to 1.2
+// The small limit also holds above 40 orbitals (n = 64, 6 references: 131072 pairs 1.04 / 2.0, 300000 pairs 0.67)
+// and with zero-overlap reference pairs (3 to 24 references: 131072 pairs 1.0 to 2.3, 300000 pairs 1.0).
 constexpr uint64_t kTileLarge = 3ull << 17;
-constexpr uint64_t kTileTables = 64ull << 20;
+constexpr uint64_t kTileTwoWaves = 2ull * 148 * 1024;
+constexpr uint64_t kTileSmall = 1ull << 17;
+constexpr int kTileLargeOrbitals = 40;
+constexpr uint64_t kTileLargeReach = 1000000;   // nref^2 n^3
 
 EvalParams make_params(const nw_ctx* ctx);
 // Number of sort keys with at most `cap` counters for the fast classes and at most gen_cap for the

@@ -101,3 +101,19 @@ def test_pinned_host_chunks(zero_pairs):
             out = torch.full((n, 2), float("nan"), dtype=torch.float64).pin_memory()
             w.eval_pairs(host.numpy().view(np.uint32), out.numpy())
             assert np.max(np.abs(out.numpy() - _both(w, torch, pairs, False)[0])) <= ROUTES, n
+
+
+@pytest.mark.parametrize("n,nref,limit", [(8, 3, 393216), (16, 8, 303104), (16, 17, 131072), (41, 2, 131072)])
+def test_route_by_references(n, nref, limit):
+    """Both sides of every line of the (H, S) size rule: the largest one-kernel request agrees with the sorted
+    pipeline, and one pair more is the sorted pipeline's own result, bit for bit."""
+    torch = pytest.importorskip("torch")
+    system = sy.make_system(n, 2, 2, nref, 2 * n, seed=3, k_scale=0.05, enuc=0.2)
+    basis = sy.sd_basis(n, 2, 2, nref)
+    with nociwick.WicksShared(system.s, system.h, system.eri, system.enuc, system.refs, tol=1e-8) as w:
+        w.build().set_basis(basis)
+        pairs = sy.sample_pairs(basis, limit + 1, seed=n, distinct_parents=False)
+        one, srt = _both(w, torch, pairs[:limit], False)
+        assert np.all(np.isfinite(one)) and np.max(np.abs(one - srt)) <= ROUTES
+        one, srt = _both(w, torch, pairs, False)
+        assert np.array_equal(one, srt)
