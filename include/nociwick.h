@@ -563,7 +563,9 @@ NW_API nw_status nw_sync(nw_ctx* ctx, void* stream);
  * device pairs (npairs of them, results into hs) for fine sort-key budgets 2^14 .. 2^23 and
  * 4 / 8 / 16 blocks per SM of the grid-stride kernels, against the defaults, and keeps the
  * fastest for the later calls on this context, the budget as keys per pair so that calls of
- * other sizes scale it (budget 0 and blocks 0 in the report mean the defaults won).
+ * other sizes scale it (budget 0 and blocks 0 in the report mean the defaults won).  Both are
+ * settings of the sorted pipeline, which every trial runs, also for pairs few enough for the
+ * one-kernel evaluation, where later calls of this size use neither.
  * Synchronises `stream`. */
 typedef struct nw_tune_report {
     uint64_t key_budget;        /* chosen fine-key budget (0: default, min(2^23, max(2^14, npairs))) */

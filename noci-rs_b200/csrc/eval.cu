@@ -725,7 +725,7 @@ nw_status eval_pairs_on(nw_ctx* ctx, EvalParams P, const uint32_t* pairs, uint64
 
   // the blocks of a blocked evaluation route like the full build
   const bool gen = any_generic(ctx);
-  if (!(ctx->timing && ctx->serial_classes) && std::max(npairs, request) <= tile_limit(P, mode, gen)) {
+  if (!(ctx->timing && ctx->serial_classes) && !ctx->tuning && std::max(npairs, request) <= tile_limit(P, mode, gen)) {
     // phase events: everything is the evaluator's
     if (ctx->timing)
       for (int i = 0; i < 4; ++i) NW_CUDA(ctx, cudaEventRecord(ctx->ev[i], stream));
@@ -870,6 +870,7 @@ nw_status eval_pairs_noalloc(nw_ctx* ctx, const uint32_t* pairs, uint64_t npairs
 // per pair so that it scales with the size of later calls
 // before evaluation: locality of the intermediates against the cost of clearing and scanning
 // the counters) and the blocks per SM of the grid-stride kernels, timed on the caller's pairs.
+// Both are settings of the sorted pipeline, so every trial runs it, whatever the size of the request.
 // ---------------------------------------------------------------------------------------
 extern "C" nw_status nw_autotune(nw_ctx* ctx, const uint32_t* pairs, uint64_t npairs, double* hs, void* stream,
                                  nw_tune_report* rep) {
@@ -891,6 +892,7 @@ extern "C" nw_status nw_autotune(nw_ctx* ctx, const uint32_t* pairs, uint64_t np
   uint64_t best_budget = 0;
   int best_per_sm = 0, trials = 0;
   nw_status st = NW_OK;
+  ctx->tuning = true;
   // (0, 0) first: the untuned defaults
   for (int b = -1; b < (int)(sizeof(kBudgets) / sizeof(kBudgets[0])) && st == NW_OK; ++b) {
     for (int g = 0; g < (int)(sizeof(kPerSm) / sizeof(kPerSm[0])) && st == NW_OK; ++g) {
@@ -917,8 +919,14 @@ extern "C" nw_status nw_autotune(nw_ctx* ctx, const uint32_t* pairs, uint64_t np
       }
     }
   }
+  ctx->tuning = false;
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  // hs holds the results of the request's own route
+  if (st == NW_OK && npairs <= nw::tile_limit(nw::make_params(ctx), nw::EvalMode::kHS, nw::any_generic(ctx))) {
+    st = nw::eval_pairs(ctx, pairs, npairs, hs, nw::EvalMode::kHS, s);
+    if (st == NW_OK && cudaStreamSynchronize(s) != cudaSuccess) st = nw::fail(ctx, NW_ERR_CUDA, "autotune results");
+  }
   if (st != NW_OK) {
     ctx->tune_keys_per_pair = saved_ratio;
     ctx->tune_per_sm = saved_per_sm;

@@ -117,3 +117,23 @@ def test_route_by_references(n, nref, limit):
         assert np.all(np.isfinite(one)) and np.max(np.abs(one - srt)) <= ROUTES
         one, srt = _both(w, torch, pairs, False)
         assert np.array_equal(one, srt)
+
+
+def test_autotune_small_request():
+    """The tuner's settings are the sorted pipeline's: on a request that the one kernel takes, a budget that only
+    clears and scans more counters (2^22 or 2^23 for 1000 pairs: 27 MB at these 6.7 10^6 keys, against 64 KB) is
+    never the fastest, and the results are the request's own."""
+    torch = pytest.importorskip("torch")
+    system = sy.make_system(40, 4, 4, 3, 80, seed=3, k_scale=0.05)
+    basis = sy.sd_basis(40, 4, 4, 3)
+    pairs = sy.sample_pairs(basis, 1000, seed=1, distinct_parents=False)
+    with nociwick.WicksShared(system.s, system.h, system.eri, system.enuc, system.refs, tol=1e-8) as w:
+        w.build().set_basis(basis)
+        one, _ = _both(w, torch, pairs, False)
+        stream = torch.cuda.current_stream().cuda_stream
+        dp = torch.from_numpy(np.ascontiguousarray(pairs.astype(np.uint32)).view(np.int32)).cuda()
+        for _ in range(8):
+            out = torch.full((1000, 2), float("nan"), dtype=torch.float64, device="cuda")
+            rep = w.autotune(dp.data_ptr(), 1000, out.data_ptr(), stream)
+            assert rep["trials"] == 19 and rep["key_budget"] < 1 << 22
+            assert np.array_equal(out.cpu().numpy(), one)
