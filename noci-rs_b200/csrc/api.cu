@@ -26,13 +26,20 @@ nw_status cuda_fail(nw_ctx* ctx, cudaError_t e, const char* what) {
 cudaError_t ctx_malloc(nw_ctx* ctx, void** p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, bytes);
   if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
   std::lock_guard<std::mutex> lock(ctx->pt2_spare->mtx);
-  DevBuf& spare = ctx->pt2_spare->buf;
-  if (spare.p) {
-    cudaGetLastError();
-    cudaFree(spare.p);
-    spare = DevBuf{};
+  DevBuf* kept[] = {&ctx->pt2_spare->buf, &ctx->pt2_table, ctx->gmres_busy ? nullptr : &ctx->gmres_work};
+  bool freed = false;
+  for (DevBuf* b : kept)
+    if (b && b->p) {
+      if (!freed) cudaDeviceSynchronize();  // kernels of earlier calls may still use them
+      cudaFree(b->p);
+      *b = DevBuf{};
+      freed = true;
+    }
+  if (freed) {
     e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();
   }
   return e;
 }
@@ -420,8 +427,8 @@ nw_status nw_set_basis(nw_ctx* ctx, const nw_det* basis, uint64_t ndet) {
   if (ndet == 0) return NW_OK;
   std::vector<uint16_t> desc(ndet);
   for (uint64_t i = 0; i < ndet; ++i) desc[i] = (uint16_t)nw::det_desc(basis[i].parent, basis[i].rank_a, basis[i].rank_b);
-  if (cudaMalloc(&ctx->d_dets, ndet * sizeof(nw_det)) != cudaSuccess ||
-      cudaMalloc(&ctx->d_desc, ndet * sizeof(uint16_t)) != cudaSuccess)
+  if (nw::ctx_malloc(ctx, reinterpret_cast<void**>(&ctx->d_dets), ndet * sizeof(nw_det)) != cudaSuccess ||
+      nw::ctx_malloc(ctx, reinterpret_cast<void**>(&ctx->d_desc), ndet * sizeof(uint16_t)) != cudaSuccess)
     return nw::fail(ctx, NW_ERR_ALLOC, "basis allocation failed");
   NW_CUDA(ctx, cudaMemcpy(ctx->d_dets, basis, ndet * sizeof(nw_det), cudaMemcpyHostToDevice));
   NW_CUDA(ctx, cudaMemcpy(ctx->d_desc, desc.data(), ndet * sizeof(uint16_t), cudaMemcpyHostToDevice));

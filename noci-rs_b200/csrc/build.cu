@@ -1085,7 +1085,7 @@ nw_status build_all(nw_ctx* ctx, const std::vector<char>* subset) {
     cudaFree(ctx->d_fbase);
     ctx->d_fbase = nullptr;
   }
-  if (cudaMalloc(&ctx->d_fbase, sizeof(double) * nps * 6 * n2) != cudaSuccess)
+  if (ctx_malloc(ctx, reinterpret_cast<void**>(&ctx->d_fbase), sizeof(double) * nps * 6 * n2) != cudaSuccess)
     return fail(ctx, NW_ERR_ALLOC, "Fock basis allocation failed");
   const double* kept[3] = {M, cx, xc};
   for (int k = 0; k < 3; ++k)
@@ -1137,12 +1137,12 @@ nw_status update_fock(nw_ctx* ctx, const double* fa, const double* fb) {
   const size_t n2 = (size_t)n * n;
   const cudaStream_t h = 0;  // the build runs on the legacy default stream
   ctx->fock_ready = false;
-  if (!ctx->d_fock && cudaMalloc(&ctx->d_fock, sizeof(double) * 2 * n2) != cudaSuccess)
+  if (!ctx->d_fock && ctx_malloc(ctx, reinterpret_cast<void**>(&ctx->d_fock), sizeof(double) * 2 * n2) != cudaSuccess)
     return fail(ctx, NW_ERR_ALLOC, "Fock matrix allocation failed");
   NW_CUDA(ctx, cudaMemcpy(ctx->d_fock, fa, sizeof(double) * n2, cudaMemcpyHostToDevice));
   NW_CUDA(ctx, cudaMemcpy(ctx->d_fock + n2, fb, sizeof(double) * n2, cudaMemcpyHostToDevice));
   double* work = nullptr;
-  if (cudaMalloc(&work, sizeof(double) * nps * 6 * n2) != cudaSuccess)
+  if (ctx_malloc(ctx, reinterpret_cast<void**>(&work), sizeof(double) * nps * 6 * n2) != cudaSuccess)
     return fail(ctx, NW_ERR_ALLOC, "Fock workspace allocation failed");
   struct Free {
     void* p;
@@ -1199,7 +1199,8 @@ nw_status update_fock(nw_ctx* ctx, const double* fa, const double* fb) {
   }
   const size_t scal_off = (slab + 3) / 4 * 4;  // FsScalars per pair, 32-byte aligned
   std::vector<FsScalars> scal(npair);
-  if (cudaMalloc(&ctx->d_fslab, sizeof(double) * scal_off + sizeof(FsScalars) * npair) != cudaSuccess)
+  if (ctx_malloc(ctx, reinterpret_cast<void**>(&ctx->d_fslab),
+                 sizeof(double) * scal_off + sizeof(FsScalars) * npair) != cudaSuccess)
     return fail(ctx, NW_ERR_ALLOC, "Fock table allocation failed");
   std::vector<FockPair> hfock(npair);
   std::memset(hfock.data(), 0, sizeof(FockPair) * npair);
@@ -1231,7 +1232,7 @@ nw_status update_fock(nw_ctx* ctx, const double* fa, const double* fb) {
   for (int p = 0; p < npair; ++p)
     scal[p] = {hfock[p].a.f0f[0], hfock[p].b.f0f[0], ctx->fast_host[p].a.pref, ctx->fast_host[p].b.pref};
   NW_CUDA(ctx, cudaMemcpy(ctx->d_fslab + scal_off, scal.data(), sizeof(FsScalars) * npair, cudaMemcpyHostToDevice));
-  if (!ctx->d_fockp && cudaMalloc(&ctx->d_fockp, sizeof(FockPair) * npair) != cudaSuccess)
+  if (!ctx->d_fockp && ctx_malloc(ctx, reinterpret_cast<void**>(&ctx->d_fockp), sizeof(FockPair) * npair) != cudaSuccess)
     return fail(ctx, NW_ERR_ALLOC, "Fock table allocation failed");
   NW_CUDA(ctx, cudaMemcpy(ctx->d_fockp, hfock.data(), sizeof(FockPair) * npair, cudaMemcpyHostToDevice));
   NW_CUDA(ctx, cudaDeviceSynchronize());

@@ -107,6 +107,7 @@ struct nw_ctx {
   nw::DevBuf pt2_scratch, pt2_table;
   std::shared_ptr<nw::SpareMatrix> pt2_spare = std::make_shared<nw::SpareMatrix>();
   nw::DevBuf gmres_work;           // vectors and scratch of the solves (kept up to kKeepGmres bytes)
+  bool gmres_busy = false;         // a solve is using them
 
   // evaluation scratch (grown on demand)
   nw::DevBuf keys, perm, counts, offsets, flag, ranks, tsum;
@@ -195,7 +196,8 @@ constexpr uint64_t kPipeTileChunk = 1ull << 16;
 nw_status fail(nw_ctx* ctx, nw_status st, const std::string& msg);
 nw_status cuda_fail(nw_ctx* ctx, cudaError_t e, const char* what);
 nw_status ensure(nw_ctx* ctx, DevBuf& b, size_t bytes);
-// cudaMalloc that gives back the context's spare candidate matrix before it fails.
+// cudaMalloc that gives back what the context keeps between candidate operators (the spare matrix, the
+// string-pair tables, the GMRES vectors outside a solve) before it fails.  Under the context's guard.
 cudaError_t ctx_malloc(nw_ctx* ctx, void** p, size_t bytes);
 
 // What a context keeps between candidate operators: allocating and freeing their matrix and vectors took

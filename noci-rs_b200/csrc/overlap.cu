@@ -710,16 +710,11 @@ nw_status overlap_plan_get(nw_ctx* ctx, cudaStream_t stream, OverlapPlan** out) 
   const size_t o_fac = carve(some(nfac) * 8), o_u = carve(some(nu) * 8);
   const size_t o_xs = carve((pl->nent + 1) * 8);
   const size_t o_t = carve((size_t)nref * nao * nmo * 8), o_o = carve(2 * nrr * n2 * 8);
-  size_t free_b = 0, total_b = 0;
-  if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && off > free_b) {
-    overlap_plan_free(pl);
-    return fail(ctx, NW_ERR_ALLOC,
-                "the overlap factor tables need " + std::to_string(off >> 20) + " MiB, more than the free device memory");
-  }
   if (ctx_malloc(ctx, reinterpret_cast<void**>(&pl->mem), off) != cudaSuccess) {
     pl->mem = nullptr;
     overlap_plan_free(pl);
-    return fail(ctx, NW_ERR_ALLOC, "overlap factor table allocation failed");
+    return fail(ctx, NW_ERR_ALLOC,
+                "the overlap factor tables need " + std::to_string(off >> 20) + " MiB, more than the free device memory");
   }
   char* base = static_cast<char*>(pl->mem);
   pl->ord_det = reinterpret_cast<uint32_t*>(base + o_det);

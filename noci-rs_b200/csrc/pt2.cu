@@ -796,17 +796,30 @@ nw_status nw_pt2_solve(nw_pt2* p, const nw_pt2_projection* proj, const double* r
   const size_t nscr = (size_t)kVBlocks * ld + 4 * (size_t)kVBlocks + 2 * (size_t)ld + (size_t)(kmax + 1) * kmax +
                       2 * (size_t)kmax + (size_t)ld;
   static_assert(sizeof(ArnoldiState) % sizeof(double) == 0, "state before the scratch");
-  if (nw::ensure(ctx, ctx->gmres_work, sizeof(double) * (n * nvec + nscr) + sizeof(ArnoldiState)) != NW_OK)
-    return pfail(p, NW_ERR_ALLOC, "GMRES vectors");
-  struct Shrink {
-    nw::DevBuf& b;
-    ~Shrink() {
+  const size_t work = sizeof(double) * (n * nvec + nscr) + sizeof(ArnoldiState);
+  nw::DevBuf& gw = ctx->gmres_work;
+  if (gw.bytes < work) {
+    // exactly what the solve needs: large vectors are not kept
+    if (gw.p) cudaFree(gw.p);
+    gw = nw::DevBuf{};
+    if (nw::ctx_malloc(ctx, &gw.p, work) != cudaSuccess) {
+      gw.p = nullptr;
+      return pfail(p, NW_ERR_ALLOC, "GMRES vectors");
+    }
+    gw.bytes = work;
+  }
+  struct Release {
+    nw_ctx* ctx;
+    ~Release() {
+      ctx->gmres_busy = false;
+      nw::DevBuf& b = ctx->gmres_work;
       if (b.bytes <= nw::kKeepGmres) return;
       cudaFree(b.p);
       b = nw::DevBuf{};
     }
-  } shrink{ctx->gmres_work};
-  double* base = static_cast<double*>(ctx->gmres_work.p);
+  } release{ctx};
+  ctx->gmres_busy = true;
+  double* base = static_cast<double*>(gw.p);
   auto vec = [&](int i) { return base + (uint64_t)i * n; };
   double *s_a0 = vec(0), *s_0a = vec(1), *f_a0 = vec(2), *f_0a = vec(3), *dinv = vec(4), *z0 = vec(5), *z1 = vec(6);
   double *b = vec(7), *x = vec(8), *r = vec(9), *w = vec(10), *z = vec(11), *Q = vec(12);

@@ -323,7 +323,7 @@ nw_status load_intermediates(nw_ctx* ctx, const char* slab_path, const char* met
     return fail(ctx, NW_ERR_ALLOC, "intermediate slab allocation failed");
   }
   ctx->slab_capacity = std::max<size_t>(hd.slab_bytes, 256);
-  if (cudaMalloc(&ctx->d_fbase, fbase_bytes) != cudaSuccess) {
+  if (ctx_malloc(ctx, reinterpret_cast<void**>(&ctx->d_fbase), fbase_bytes) != cudaSuccess) {
     ctx->d_fbase = nullptr;
     return fail(ctx, NW_ERR_ALLOC, "Fock basis allocation failed");
   }
