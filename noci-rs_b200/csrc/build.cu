@@ -622,13 +622,16 @@ nw_status build_all(nw_ctx* ctx, const std::vector<char>* subset) {
                         4 * n2 /*X Y*/ + 2 * n2 /*tmp*/ + 2 * n2 /*JK*/ + 2 * n2 /*Jc*/ + 4 * n2 /*Fh*/ +
                         8 * n2 /*V*/ + 8 * n2 /*vab or vba*/ + 2 * n2 /*hxc*/ + 4 * n2 /*JKxc*/ +
                         4 * n2 /*JcXc*/ + 64;
-  const int nhalf_max = 16 * npair;  // first halves of the fused transforms, all pairs
-  const size_t half = n2 * packed_ld(n);
-  // the fused transforms hold at least eight first halves (half a tensor each) and one whole tensor; a
-  // small system holds them all, so that each stage is one launch
-  const size_t tensor_work = std::max<size_t>(8 * half + n4, std::min<size_t>(nhalf_max * half + n4, 8u << 20));
+  // Four-index scratch beside G: three tensors of the quarter-transform route (and the scratch of the J / K
+  // products), or for the fused transforms at least eight first halves (half a tensor each) and one whole
+  // tensor; a small system holds all first halves, so that each stage is one launch.
+  const bool may_fuse = ctx->transform == NW_TRANSFORM_FP64 && n <= kTwoSidedMax && ctx->eri_symmetric != 0;
+  const size_t half = n2 * packed_ld(n), nhalf_max = 16 * (size_t)npair;
+  size_t tensors = 4 * n4 + 128;
+  if (may_fuse)
+    tensors = std::max(tensors, std::max<size_t>(8 * half + n4, std::min<size_t>(nhalf_max * half + n4, 8u << 20)));
   // 40 arena pieces, each rounded up to 256 bytes
-  const size_t work_doubles = per_ps * nps + n4 + std::max<size_t>(4 * n4 + 128, tensor_work) + 40 * 32 + 4096;
+  const size_t work_doubles = per_ps * nps + n4 + tensors + 40 * 32 + 4096;
   // the workspace stays with the context, so rebuilds (blocked evaluation, transform changes)
   // do not allocate it again
   Arena ar;
@@ -668,8 +671,6 @@ nw_status build_all(nw_ctx* ctx, const std::vector<char>* subset) {
   double* JKxc = ar.take((size_t)nps * 4 * n2);
   double* JcXc = ar.take((size_t)nps * 4 * n2);
   double* G = ar.take(n4);
-  // four-index scratch: three tensors of the quarter-transform route, or the first halves of the fused one
-  const size_t tensors = std::max<size_t>(4 * n4 + 128, tensor_work);
   double* tA = ar.take(tensors);
   if (!tA) return fail(ctx, NW_ERR_ALLOC, "build workspace too small");
   const size_t n4r = (n4 + 31) / 32 * 32;
@@ -678,12 +679,12 @@ nw_status build_all(nw_ctx* ctx, const std::vector<char>* subset) {
   // Route of the four-index tensors.  The fused half transforms need the tensor's permutation symmetry
   // (checked once per context, to rounding: 32 ulp of the largest element) and n <= kTwoSidedMax, the
   // matrices that fit shared memory; otherwise the quarter transforms (or a Cholesky route) run.
-  if (ctx->transform == NW_TRANSFORM_FP64 && ctx->eri_symmetric < 0) {
+  if (may_fuse && ctx->eri_symmetric < 0) {
     double big = 0.0, off = 0.0;
     NW_CUDA(ctx, eri_symmetry(h, ctx->d_eri, n, G, &big, &off));
     ctx->eri_symmetric = off <= 32 * 2.220446049250313e-16 * big ? 1 : 0;
   }
-  const bool fused = ctx->transform == NW_TRANSFORM_FP64 && n <= kTwoSidedMax && ctx->eri_symmetric == 1;
+  const bool fused = may_fuse && ctx->eri_symmetric == 1;
   // Cholesky route of the four-index tensors (nw_set_transform)
   CholWork cw{};
   CholWork* cwp = nullptr;

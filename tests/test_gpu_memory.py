@@ -54,3 +54,18 @@ def test_kept_operator_memory_is_given_back():
             torch.cuda.empty_cache()
     # chunks of a long row are added by atomics, in no fixed order
     assert float((got - want).abs().max()) <= 1e-11 * float(want.abs().max())
+
+
+def test_build_scratch_beyond_the_fused_transforms():
+    """Above 64 orbitals a build takes three tensors a reference pair and a workspace of five (grown by a
+    quarter), beside matrices of n^2 and what the driver rounds up; the context's own memory is not counted."""
+    torch = pytest.importorskip("torch")
+    n = 72
+    system = sy.make_system(n, 2, 2, 1, 2 * n, seed=4)
+    for _ in range(2):              # the first one loads the kernels
+        with nociwick.WicksShared(system.s, system.h, system.eri, system.enuc, system.refs, tol=1e-8) as w:
+            torch.cuda.synchronize()
+            before = torch.cuda.mem_get_info()[0]
+            w.build()
+            used = before - torch.cuda.mem_get_info()[0]
+    assert used <= 8 * n ** 4 * (3 + 1.25 * 5) + (64 << 20)
