@@ -134,6 +134,8 @@ nw_status build_matrix(nw_ctx* ctx, EvalMode mode, const uint32_t* left, uint64_
   if ((st = dev_alloc(ctx, dpairs, cap * sizeof(uint2), "pair block")) != NW_OK) return st;
   if ((st = dev_alloc(ctx, dvals, cap * 2 * sizeof(double), "pair values")) != NW_OK) return st;
   if ((st = dev_alloc(ctx, doff, std::min<uint64_t>(nl, cap) * sizeof(uint64_t), "row offsets")) != NW_OK) return st;
+  // every block takes the whole matrix's route
+  const uint64_t request = symmetric ? nl * (nl + 1) / 2 : nl * nr;
   std::vector<uint64_t> off;
   uint64_t r0 = 0;
   while (r0 < nl) {
@@ -151,7 +153,8 @@ nw_status build_matrix(nw_ctx* ctx, EvalMode mode, const uint32_t* left, uint64_
     matrix_pairs_kernel<<<(unsigned)nrow, 256>>>(dl.as<uint32_t>(), dr.as<uint32_t>(), r0, nr, symmetric ? 1 : 0,
                                                  doff.as<uint64_t>(), dpairs.as<uint2>());
     NW_CUDA(ctx, cudaGetLastError());
-    if ((st = eval_pairs(ctx, dpairs.as<uint32_t>(), total, dvals.as<double>(), mode, nullptr)) != NW_OK) return st;
+    if ((st = eval_pairs(ctx, dpairs.as<uint32_t>(), total, dvals.as<double>(), mode, nullptr, true, request)) != NW_OK)
+      return st;
     matrix_scatter_kernel<<<(unsigned)nrow, 256>>>(dvals.as<double2>(), r0, nr, symmetric ? 1 : 0,
                                                    doff.as<uint64_t>(), da.as<double>(), ds.as<double>());
     NW_CUDA(ctx, cudaGetLastError());

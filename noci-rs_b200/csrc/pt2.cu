@@ -568,7 +568,8 @@ nw_status symv(nw_pt2* p, const double* x, double* y) {
     const uint64_t nt = std::min(per_block, ntiles - t0), nslots = nt * kTileSlots;
     tile_pairs_kernel<<<grid_n(nslots), 256>>>(p->dcand, n, nb, t0, nslots, p->pairs);
     nw_status st = nw::eval_pairs(p->ctx, reinterpret_cast<const uint32_t*>(p->pairs), nslots,
-                                  reinterpret_cast<double*>(p->fs), nw::EvalMode::kFS, nullptr);
+                                  reinterpret_cast<double*>(p->fs), nw::EvalMode::kFS, nullptr, true,
+                                  ntiles * kTileSlots);
     if (st != NW_OK) return st;
     mf_tile_apply_kernel<<<(unsigned)nt, kTile>>>(p->fs, n, nb, t0, p->e0, x, y);
     NW_CUDA(p->ctx, cudaGetLastError());
@@ -692,7 +693,7 @@ nw_status nw_pt2_create(nw_ctx* ctx, const uint32_t* cand, uint64_t n, double e0
     const uint64_t count = std::min(blk, len - base);
     upper_pairs_kernel<<<grid_n(count), 256>>>(dcand, n, base, count, pairs);
     nw_status st = nw::eval_pairs(ctx, reinterpret_cast<const uint32_t*>(pairs), count, reinterpret_cast<double*>(fs),
-                                  nw::EvalMode::kFS, nullptr);
+                                  nw::EvalMode::kFS, nullptr, true, len);
     if (st != NW_OK) return cleanup(st);
     packed_fill_kernel<<<grid_n(count), 256>>>(fs, count, e0, p->m + base);
     if (cudaGetLastError() != cudaSuccess) return cleanup(nw::fail(ctx, NW_ERR_CUDA, "packed fill"));

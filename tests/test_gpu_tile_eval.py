@@ -137,3 +137,26 @@ def test_autotune_small_request():
             rep = w.autotune(dp.data_ptr(), 1000, out.data_ptr(), stream)
             assert rep["trials"] == 19 and rep["key_budget"] < 1 << 22
             assert np.array_equal(out.cpu().numpy(), one)
+
+
+@pytest.mark.parametrize("fs", [False, True])
+def test_blocks_of_a_matrix_take_one_route(fs):
+    """A dense matrix in row blocks of 2^24 pairs, the last one small: every element as the device call gives it
+    for all pairs at once, bit for bit, with zero-overlap reference pairs."""
+    torch = pytest.importorskip("torch")
+    system = sy.make_system(8, 3, 3, 3, 20, seed=1, k_scale=0.3, zero_pairs=[(0, 1, 1, 0)], enuc=0.37)
+    basis = sy.sd_basis(8, 3, 3, 3)
+    rng = np.random.default_rng(3)
+    left, right = (rng.integers(0, basis.shape[0], 4100).astype(np.uint32) for _ in range(2))
+    with nociwick.WicksShared(system.s, system.h, system.eri, system.enuc, system.refs, tol=1e-8) as w:
+        w.build().set_basis(basis)
+        w.update_fock(system.h, system.h)
+        got = (w.build_fs_matrix if fs else w.build_hs_matrix)(left, right, symmetric=False)
+        pairs = np.stack([np.repeat(left, 4100), np.tile(right, 4100)], axis=1)
+        dp = torch.from_numpy(pairs.view(np.int32)).cuda()
+        out = torch.empty((pairs.shape[0], 2), dtype=torch.float64, device="cuda")
+        stream = torch.cuda.current_stream().cuda_stream
+        (w.eval_fs_pairs_device if fs else w.eval_pairs_device)(dp.data_ptr(), pairs.shape[0], out.data_ptr(), stream)
+        w.sync(stream)
+        want = out.cpu().numpy().reshape(4100, 4100, 2)
+    assert np.array_equal(got[0], want[:, :, 0]) and np.array_equal(got[1], want[:, :, 1])
