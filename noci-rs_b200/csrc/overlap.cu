@@ -70,7 +70,6 @@ struct OvlTile {
   uint64_t x0;      // kOvlTile source entries per table row (the last entry + 1: none)
   uint32_t k0, nk;  // table rows
   uint32_t nrow, ld;
-  uint32_t atomic, pad;
 };
 // One source of a row: table row and position among the distinct (parent, a, b) entries.
 struct OvlSource {
@@ -95,31 +94,28 @@ constexpr uint32_t kOvlTileK = 160;   // table rows of a dense tile held at once
 constexpr uint32_t kOvlTargets = 64;  // targets of a stage-2 block (kOvlThreads / kOvlTargets term segments)
 constexpr uint64_t kOvlWork = 1ull << 27;  // doubles of U and W per batch of target parents (1 GB)
 
-// One entry of a single-spin factor table per thread; MAXO bounds nocc (the LU scratch lives in
+// One entry of a (source-major) single-spin factor table per thread; MAXO bounds nocc (the LU scratch lives in
 // the thread's stack frame, MAXO^2 doubles).
 template <int MAXO>
 __global__ void __launch_bounds__(kOvlThreads) ovl_factor_kernel(const double* __restrict__ o, int nmo,
                                                                   const uint8_t* __restrict__ occ_t,
                                                                   const uint8_t* __restrict__ occ_s, int nocc,
-                                                                  uint32_t nt, uint32_t ns, int source_major,
-                                                                  uint32_t ld, double* __restrict__ out) {
+                                                                  uint32_t nt, uint32_t ns, uint32_t ld,
+                                                                  double* __restrict__ out) {
   const uint64_t total = (uint64_t)nt * ns;
   for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < total; e += (uint64_t)gridDim.x * blockDim.x) {
     // consecutive threads write consecutive entries of the output row
-    const uint32_t i = source_major ? (uint32_t)(e % nt) : (uint32_t)(e / ns);
-    const uint32_t j = source_major ? (uint32_t)(e / nt) : (uint32_t)(e % ns);
+    const uint32_t i = (uint32_t)(e % nt), j = (uint32_t)(e / nt);
     const uint8_t* oi = occ_t + (uint64_t)i * nocc;
     const uint8_t* oj = occ_s + (uint64_t)j * nocc;
     double m[MAXO * MAXO];
     for (int r = 0; r < nocc; ++r)
       for (int c = 0; c < nocc; ++c) m[r * nocc + c] = o[(uint64_t)oi[r] * nmo + oj[c]];
-    const double d = det_lu_inplace(m, nocc);
-    out[source_major ? (uint64_t)j * ld + i : (uint64_t)i * ns + j] = d;
+    out[(uint64_t)j * ld + i] = det_lu_inplace(m, nocc);
   }
 }
 
-// xs[e] = sum of r x over the determinants of distinct entry e (xs[nent] = 0 stands for no source), and
-// zeros in the output rows that several chunks add into.
+// xs[e] = sum of r x over the determinants of distinct entry e (xs[nent] = 0 stands for no source).
 __global__ void __launch_bounds__(kOvlThreads) ovl_gather_kernel(uint64_t nent, const uint32_t* __restrict__ first,
                                                                   const uint32_t* __restrict__ ord_det,
                                                                   const double* __restrict__ ord_r,
@@ -133,6 +129,7 @@ __global__ void __launch_bounds__(kOvlThreads) ovl_gather_kernel(uint64_t nent, 
   }
 }
 
+// Zeros in the output rows that several chunks add into.
 __global__ void __launch_bounds__(kOvlThreads) ovl_zero_kernel(const ulonglong2* __restrict__ rows,
                                                                 double* __restrict__ u) {
   const ulonglong2 r = rows[blockIdx.x];  // offset, length
@@ -655,7 +652,7 @@ nw_status overlap_plan_get(nw_ctx* ctx, cudaStream_t stream, OverlapPlan** out) 
           for (const Shape& sh : side ? cshape[p] : rshape[p]) {
             const uint64_t out = uq + (uint64_t)sh.l0 * ld;
             if (sh.tile) {
-              tiles.push_back(OvlTile{tab, out, sh.x0, sh.k0, sh.nk, sh.nl, ld, 0u, 0u});
+              tiles.push_back(OvlTile{tab, out, sh.x0, sh.k0, sh.nk, sh.nl, ld});
               continue;
             }
             const bool multi = sh.nk > kOvlChunk;
@@ -778,11 +775,11 @@ nw_status overlap_plan_get(nw_ctx* ctx, cudaStream_t stream, OverlapPlan** out) 
     const uint64_t e = (uint64_t)nt * ns;
     if (e == 0) return;
     if (nocc <= 4)
-      ovl_factor_kernel<4><<<grid_of(e), kOvlThreads, 0, stream>>>(o, nmo, ot, os, nocc, nt, ns, 1, ld, out);
+      ovl_factor_kernel<4><<<grid_of(e), kOvlThreads, 0, stream>>>(o, nmo, ot, os, nocc, nt, ns, ld, out);
     else if (nocc <= 8)
-      ovl_factor_kernel<8><<<grid_of(e), kOvlThreads, 0, stream>>>(o, nmo, ot, os, nocc, nt, ns, 1, ld, out);
+      ovl_factor_kernel<8><<<grid_of(e), kOvlThreads, 0, stream>>>(o, nmo, ot, os, nocc, nt, ns, ld, out);
     else
-      ovl_factor_kernel<kOvlMaxOcc><<<grid_of(e), kOvlThreads, 0, stream>>>(o, nmo, ot, os, nocc, nt, ns, 1, ld, out);
+      ovl_factor_kernel<kOvlMaxOcc><<<grid_of(e), kOvlThreads, 0, stream>>>(o, nmo, ot, os, nocc, nt, ns, ld, out);
   };
   for (int q = 0; ok && q < nref; ++q)
     for (int p = 0; ok && p < nref; ++p) {
