@@ -113,3 +113,31 @@ def test_operator_outlives_its_context():
     pt = nociwick.Pt2(w, np.arange(1200, dtype=np.uint32), -0.5)
     w.close()
     pt.close()
+
+
+def test_rows_beyond_shared_memory():
+    """More strings than a staged pair of table rows holds (220 KB: 14080 strings of both spins): columns of M
+    against the elements of the pair evaluation, which agree to a few roundings of terms of order 10."""
+    system = sy.make_system(28, 9, 9, 3, 112, seed=2, sigma_h=0.02, sigma_l=0.02, k_scale=0.3, uhf_like=True)
+    basis = sy.sd_basis(28, 9, 9, 3)
+    rng = np.random.default_rng(6)
+    kinds = [((2, 0), 6900), ((0, 2), 6900), ((1, 1), 16200)]
+    cand = np.concatenate([rng.choice(np.nonzero((basis["rank_a"] == a) & (basis["rank_b"] == b))[0], k, replace=False)
+                           for (a, b), k in kinds])
+    cand = rng.permutation(cand).astype(np.uint32)
+    n = cand.shape[0]
+    strings = [len({(int(d["parent"]), int(d[r]), d[i].tobytes()) for d in basis[cand]})
+               for r, i in (("rank_a", "idx_a"), ("rank_b", "idx_b"))]
+    assert sum(strings) > 14080 and strings[0] ** 2 + strings[1] ** 2 <= n * (n + 1) // 8
+    e0 = -0.75
+    with nociwick.WicksShared(system.s, system.h, system.eri, system.enuc, system.refs, tol=1e-8) as w:
+        w.build().set_basis(basis)
+        w.update_fock(*sy.reference_fock(system, 0))
+        with nociwick.Pt2(w, cand, e0) as pt:
+            for k in (0, 1, n // 2, n - 2, n - 1):
+                x = np.zeros(n)
+                x[k] = 1.0
+                pos = np.arange(n)
+                pairs = np.stack([cand[np.minimum(pos, k)], cand[np.maximum(pos, k)]], axis=1)
+                fs = w.eval_fs_pairs(pairs)
+                assert np.max(np.abs(pt.apply_m(x) - (fs[:, 0] - e0 * fs[:, 1]))) <= 1e-12
