@@ -111,7 +111,7 @@ struct nw_ctx {
 
   // evaluation scratch (grown on demand)
   nw::DevBuf keys, perm, counts, offsets, flag, ranks, tsum;
-  uint32_t* h_flag = nullptr;      // pinned: mirror of the device error flag; words 4, 5: GMRES steps
+  uint32_t* h_flag = nullptr;      // pinned: mirror of the device error flag; word 4: the GMRES cycle is done
   nw::DevBuf io_pairs, io_hs;      // staging for the host-buffer entry point
   // determinant records, descriptors and pairs packed from caller excitation caches
   // (nw_eval_hs_batched), and their device staging for host-buffer calls

@@ -141,3 +141,28 @@ def test_rows_beyond_shared_memory():
                 pairs = np.stack([cand[np.minimum(pos, k)], cand[np.maximum(pos, k)]], axis=1)
                 fs = w.eval_fs_pairs(pairs)
                 assert np.max(np.abs(pt.apply_m(x) - (fs[:, 0] - e0 * fs[:, 1]))) <= 1e-12
+
+
+@pytest.mark.parametrize("restart", [4, 7, 40])
+def test_long_solves_replay_the_step(restart):
+    """Solves beyond the plain steps, in one cycle and over several (the step is replayed as a graph), against the
+    matrix-free operator, whose steps are always launched one by one; a second solve starts afresh."""
+    system = sy.make_system(12, 4, 3, 3, 40, seed=2, k_scale=0.3)
+    basis = sy.sd_basis(12, 4, 3, 3)
+    rng = np.random.default_rng(4)
+    cand = rng.choice(basis.shape[0], 1300, replace=False).astype(np.uint32)
+    vecs = [0.01 * rng.normal(size=1300) for _ in range(5)]
+    with nociwick.WicksShared(system.s, system.h, system.eri, system.enuc, system.refs, tol=1e-8) as w:
+        w.build().set_basis(basis)
+        w.update_fock(system.h, system.h)
+        for max_iter in (5, 6, 7, 20, 41):
+            got = []
+            for free in (False, True):
+                with nociwick.Pt2(w, cand, -30.0, matrix_free=free) as pt:
+                    a = pt.solve(-30.0, *vecs, max_iter=max_iter, restart=restart, res_tol=1e-13)
+                    b = pt.solve(-30.0, *vecs, max_iter=max_iter, restart=restart, res_tol=1e-13)
+                assert a[1]["iterations"] == b[1]["iterations"]
+                got += [a[0], b[0]]
+            scale = max(1.0, np.max(np.abs(got[2])))
+            for x in got:
+                assert np.max(np.abs(x - got[2])) <= 1e-9 * scale
