@@ -417,6 +417,7 @@ void split_sources(const std::vector<uint32_t>& ea, const std::vector<uint32_t>&
     }
   }
   std::vector<std::vector<OvlSource>> lr(na), lc(nb);
+  // entries come in (a, b) order, so every line's list is in table-row order
   for (size_t e = 0; e < ne; ++e) {
     if (by_row(best, e))
       lr[ea[e]].push_back(OvlSource{eb[e], (uint32_t)(e0 + e)});
@@ -431,7 +432,6 @@ void split_sources(const std::vector<uint32_t>& ea, const std::vector<uint32_t>&
     std::stable_sort(id.begin(), id.end(), [&](uint32_t x, uint32_t y) { return l[x].size() > l[y].size(); });
     for (uint32_t i : id) {
       out->id.push_back(i);
-      std::sort(l[i].begin(), l[i].end(), [](const OvlSource& x, const OvlSource& y) { return x.row < y.row; });
       out->src.push_back(std::move(l[i]));
     }
   };
@@ -582,29 +582,32 @@ nw_status overlap_plan_get(nw_ctx* ctx, cudaStream_t stream, OverlapPlan** out) 
     uint32_t k0, nk;     // tile: table rows; line: sources in `src`
     uint64_t x0;
   };
-  auto shapes_of = [&](const Lines& L) {
+  auto shapes_of = [&](const Lines& L, uint32_t nrows) {
     std::vector<Shape> out;
+    std::vector<uint32_t> rows, seen(nrows, 0), place(nrows);  // distinct table rows of a window of lines
+    uint32_t window = 0;
     for (uint32_t l = 0; l < L.id.size();) {
       // a tile where the lines share their entries: at most 1.5 times the work of the lines one by one
       const uint32_t nl = std::min<uint32_t>(kOvlTile, (uint32_t)L.id.size() - l);
-      std::vector<uint32_t> rows;
+      rows.clear();
+      ++window;
       uint64_t nnz = 0;
-      for (uint32_t i = 0; i < nl; ++i)
-        for (const OvlSource& s : L.src[l + i]) {
-          rows.push_back(s.row);
-          ++nnz;
-        }
-      std::sort(rows.begin(), rows.end());
-      rows.erase(std::unique(rows.begin(), rows.end()), rows.end());
+      for (uint32_t i = 0; i < nl; ++i) {
+        nnz += L.src[l + i].size();
+        for (const OvlSource& s : L.src[l + i])
+          if (seen[s.row] != window) {
+            seen[s.row] = window;
+            rows.push_back(s.row);
+          }
+      }
       if (nl >= 4 && 2 * rows.size() * nl <= 3 * nnz) {
+        std::sort(rows.begin(), rows.end());
+        for (uint32_t k = 0; k < rows.size(); ++k) place[rows[k]] = k;
         const Shape sh{true, l, nl, (uint32_t)trow.size(), (uint32_t)rows.size(), tent.size()};
         trow.insert(trow.end(), rows.begin(), rows.end());
         tent.resize(sh.x0 + rows.size() * kOvlTile, (uint32_t)pl->nent);
         for (uint32_t i = 0; i < nl; ++i)
-          for (const OvlSource& s : L.src[l + i]) {
-            const size_t k = std::lower_bound(rows.begin(), rows.end(), s.row) - rows.begin();
-            tent[sh.x0 + k * kOvlTile + i] = s.entry;
-          }
+          for (const OvlSource& s : L.src[l + i]) tent[sh.x0 + (uint64_t)place[s.row] * kOvlTile + i] = s.entry;
         out.push_back(sh);
         l += nl;
       } else {
@@ -617,8 +620,8 @@ nw_status overlap_plan_get(nw_ctx* ctx, cudaStream_t stream, OverlapPlan** out) 
   };
   std::vector<std::vector<Shape>> rshape(nref), cshape(nref);
   for (int p = 0; p < nref; ++p) {
-    rshape[p] = shapes_of(R[p]);
-    cshape[p] = shapes_of(C[p]);
+    rshape[p] = shapes_of(R[p], pl->nb[p]);
+    cshape[p] = shapes_of(C[p], pl->na[p]);
   }
   auto work_of = [&](int q) {
     uint64_t w = 0;
