@@ -86,6 +86,7 @@ nw_status eval_batched(nw_ctx* ctx, EvalMode mode, int lp, int gp, const nw_exc_
   P.dets = dets;
   P.desc = desc;
   P.ndet = 2 * n;
+  P.span = 1;  // the tables of one reference pair
   return eval_pairs_on(ctx, P, reinterpret_cast<const uint32_t*>(pairs), n, hs, mode, s);
 }
 

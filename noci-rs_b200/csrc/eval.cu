@@ -495,6 +495,7 @@ EvalParams make_params(const nw_ctx* ctx) {
   P.fslab = ctx->d_fslab;
   P.nbucket = 1;
   P.shift = 0;
+  P.span = ctx->nref;
   P.ngsub = 1;
   P.gshift = 32;
   return P;

@@ -36,6 +36,7 @@ struct EvalParams {
   const double* fslab;     // their slab: 8 n^2 doubles per ordered pair, then FsScalars per pair
   uint32_t nbucket;        // sort keys per rank class for fast pairs (pair_sort_key)
   int32_t shift;
+  int32_t span;            // references that the request's pairs can belong to (its route)
   uint32_t ngsub;          // bra sub-buckets of a zero-overlap class
   int32_t gshift;
   double enuc, tol;
@@ -328,7 +329,7 @@ constexpr uint64_t kFineMin = 1ull << 14;
 // Largest (H, S) requests that take the one-kernel evaluation (tile_eval.cu); the sorted pipeline's order pays
 // for larger ones.  A tile of unordered pairs reads the tables of every reference pair, so the line falls as
 // references are added; between 12 and 40 orbitals it follows nref^2 n^3 (singles and doubles, 2 to 48
-// references).  Time of the sorted pipeline over the one kernel's, for uniform pairs of all references and of
+// references; a call for one reference pair counts one).  Time of the sorted pipeline over the one kernel's, for uniform pairs of all references and of
 // different ones / for pairs whose total rank is uniform over 0..4:
 //   nref^2 n^3 <= 10^6 (3 references to n = 40, 5 at n = 30, 8 at n = 24, 24 at n = 12)
 //       300000 pairs 0.94 to 1.74 (one kernel: two waves of tiles), 350000 pairs 0.82 to 1.26;

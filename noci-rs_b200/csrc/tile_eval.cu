@@ -284,9 +284,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) hs_tile_kernel(const __grid_c
 
 uint64_t tile_limit(const EvalParams& P, EvalMode mode, bool gen) {
   if (mode == EvalMode::kFS) return gen ? kTileSmall : ~0ull;
-  const uint64_t reach = (uint64_t)P.nref * P.nref * P.n * P.n * P.n;
+  const uint64_t reach = (uint64_t)P.span * P.span * P.n * P.n * P.n;
   if (gen || P.n > kTileLargeOrbitals || reach > kTileLargeReach) return kTileSmall;
-  return P.nref <= 3 ? kTileLarge : kTileTwoWaves;
+  return P.span <= 3 ? kTileLarge : kTileTwoWaves;
 }
 
 cudaError_t eval_tiles(const EvalParams& P, const uint2* pairs, uint64_t npairs, double* out, EvalMode mode, bool gen,
