@@ -160,3 +160,20 @@ def test_blocks_of_a_matrix_take_one_route(fs):
         w.sync(stream)
         want = out.cpu().numpy().reshape(4100, 4100, 2)
     assert np.array_equal(got[0], want[:, :, 0]) and np.array_equal(got[1], want[:, :, 1])
+
+
+def test_one_reference_pair_among_many():
+    """A request for one reference pair in a context of many keeps the one kernel where pairs of all references are
+    sorted: both give the same elements."""
+    torch = pytest.importorskip("torch")
+    system = sy.make_system(16, 2, 2, 20, 32, seed=3, k_scale=0.05, enuc=0.2)
+    basis = sy.sd_basis(16, 2, 2, 20)
+    per = basis.shape[0] // 20
+    rng = np.random.default_rng(7)
+    i, j = 3 * per + rng.integers(0, per, 140000), 11 * per + rng.integers(0, per, 140000)
+    exc = nociwick.lib.exc_caches(basis)
+    with nociwick.WicksShared(system.s, system.h, system.eri, system.enuc, system.refs, tol=1e-8) as w:
+        w.build().set_basis(basis)
+        got = w.eval_batched(3, 11, exc[i], exc[j], basis["phase"][i] * basis["phase"][j])
+        want = _both(w, torch, np.stack([i, j], axis=1), False)[1]
+    assert np.all(np.isfinite(got)) and np.max(np.abs(got - want)) <= ROUTES
